@@ -113,24 +113,31 @@ ZK_HD uint64_t gl_reduce96(uint64_t lo, uint64_t hi) { return gl_canon(gl_reduce
 // ------------------------------------------------------------------------
 // Lazily reduced arithmetic ("nc" = any 64-bit representative, not
 // necessarily < p).  On the device these are 32-bit PTX carry chains: the
-// 64x64 product is 8 multiply-adds, the reduction of lo + 2^64*(h0 + 2^32*h1)
+// 64x64 product is four wide multiply-adds, the reduction of lo + 2^64*(h0 + 2^32*h1)
 // to lo - h1 + EPS*h0 is one wide multiply and 10 integer ops (or 13 integer
 // ops in the all-ALU form) with no compares or selects.
 
 #ifdef __CUDACC__
+// The middle products are summed in one aligned register pair, so the four
+// wide multiply-adds need no register moves.
 __device__ __forceinline__ void mul_wide(uint64_t a, uint64_t b, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3)
 {
     const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
     asm("{\n\t"
-        "mul.lo.u32      %0, %4, %6;\n\t"
-        "mul.hi.u32      %1, %4, %6;\n\t"
-        "mad.lo.cc.u32   %1, %5, %6, %1;\n\t"
-        "madc.hi.u32     %2, %5, %6, 0;\n\t"
-        "mad.lo.cc.u32   %1, %4, %7, %1;\n\t"
-        "madc.hi.cc.u32  %2, %4, %7, %2;\n\t"
-        "addc.u32        %3, 0, 0;\n\t"
-        "mad.lo.cc.u32   %2, %5, %7, %2;\n\t"
-        "madc.hi.u32     %3, %5, %7, %3;\n\t"
+        ".reg .u64 p00, p01, p11;\n\t"
+        ".reg .u32 h0, q0, q1, l2, h2, m0, m1;\n\t"
+        "mul.wide.u32    p00, %4, %6;\n\t"
+        "mul.wide.u32    p01, %4, %7;\n\t"
+        "mul.wide.u32    p11, %5, %7;\n\t"
+        "mov.b64         {%0, h0}, p00;\n\t"
+        "mov.b64         {q0, q1}, p01;\n\t"
+        "mov.b64         {l2, h2}, p11;\n\t"
+        "mad.lo.cc.u32   m0, %5, %6, q0;\n\t"
+        "madc.hi.cc.u32  m1, %5, %6, q1;\n\t"
+        "addc.u32        h2, h2, 0;\n\t"
+        "add.cc.u32      %1, h0, m0;\n\t"
+        "addc.cc.u32     %2, l2, m1;\n\t"
+        "addc.u32        %3, h2, 0;\n\t"
         "}"
         : "=&r"(r0), "=&r"(r1), "=&r"(r2), "=&r"(r3)
         : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
@@ -184,34 +191,31 @@ __device__ __forceinline__ uint64_t reduce_nc_alu(uint32_t r0, uint32_t r1, uint
     return ((uint64_t)t1 << 32) | t0;
 }
 
-// The same reduction with r2 * EPS taken by one wide multiply (the multiply
-// pipe) and three fewer ALU instructions: (top:t) = (r1:r0) + r2 * EPS - r3
-// with a signed top limb in {-1, 0, 1}, then one correction t + top * EPS
-// (2^64 = EPS mod p; +EPS cannot wrap again because t <= 2^64 - 2^33 when
-// top = 1, and t >= 2^64 - 2^32 when top = -1).  The default of the lazy
-// products below: measured 1.03-1.05x on the Poseidon, Poseidon2 and Monolith
-// forests and 1.02-1.03x on the NTT passes on B200, whose integer ALU is the
-// busier pipe in all of them (the all-ALU form stays for comparison and the
-// multiply-rate probe).
+// The same reduction with r2 * EPS taken by one wide multiply-add (the
+// multiply pipe): r3 is subtracted first, top = -borrow, then r2 * EPS added
+// with its carry into top, and one correction t + top * EPS, top in {-1, 0, 1}
+// (2^64 = EPS mod p; it cannot wrap again: when top = 1, t <= 2^64 - 2^33; when
+// top = -1, the subtraction borrowed, so t >= 2^64 - EPS).  With the borrow
+// taken first its register doubles as the carry's: 16.05 instructions a
+// product, 1327 Gmul/s in a loop of S-boxes on B200, against 17.25 and 1236
+// with the subtraction after the fold, and 18.3 and 1110 all on the ALU.
 __device__ __forceinline__ uint64_t reduce_nc_imad(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3)
 {
-    uint64_t e;
-    asm("mul.wide.u32 %0, %1, 0xffffffff;" : "=l"(e) : "r"(r2));
     uint32_t t0, t1, top, cl, ch;
     asm("{\n\t"
-        "add.cc.u32      %0, %5, %7;\n\t"   // t = lo + r2 * EPS
-        "addc.cc.u32     %1, %6, %8;\n\t"
-        "addc.u32        %2, 0, 0;\n\t"
-        "sub.cc.u32      %0, %0, %9;\n\t"   // - r3
-        "subc.cc.u32     %1, %1, 0;\n\t"
-        "subc.u32        %2, %2, 0;\n\t"    // top in {-1, 0, 1}
+        "sub.cc.u32      %0, %5, %8;\n\t"   // t = lo - r3, top = -borrow
+        "subc.cc.u32     %1, %6, 0;\n\t"
+        "subc.u32        %2, 0, 0;\n\t"
+        "mad.lo.cc.u32   %0, %7, 0xffffffff, %0;\n\t"  // t += r2 * EPS
+        "madc.hi.cc.u32  %1, %7, 0xffffffff, %1;\n\t"
+        "addc.u32        %2, %2, 0;\n\t"    // top in {-1, 0, 1}
         "neg.s32         %3, %2;\n\t"       // top * EPS mod 2^64 = (-top) + 2^32 * (top >> 31)
         "shr.s32         %4, %2, 31;\n\t"
         "add.cc.u32      %0, %0, %3;\n\t"
         "addc.u32        %1, %1, %4;\n\t"
         "}"
         : "=&r"(t0), "=&r"(t1), "=&r"(top), "=&r"(cl), "=&r"(ch)
-        : "r"(r0), "r"(r1), "r"((uint32_t)e), "r"((uint32_t)(e >> 32)), "r"(r3));
+        : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
     return ((uint64_t)t1 << 32) | t0;
 }
 
@@ -294,6 +298,17 @@ struct WideAcc {
 #else
         lo = hi = 0;
         top = 0;
+#endif
+    }
+    // = x
+    ZK_HD void start(uint64_t x)
+    {
+        zero();
+#ifdef __CUDA_ARCH__
+        r0 = (uint32_t)x;
+        r1 = (uint32_t)(x >> 32);
+#else
+        lo = x;
 #endif
     }
     // += a * b (any 64-bit representatives)
