@@ -268,8 +268,9 @@ RustError zeknox_field_selftest(size_t device_id, const uint64_t *a, const uint6
 /* One permutation of each of n states, in place: 12-word states for Poseidon
  * (0), Poseidon-BN128 (2), Poseidon2 (3) and Monolith (4), lanes any 64-bit
  * words in and canonical out; 25-word Keccak-f[1600] states for Keccak (1).
- * cooperative != 0 runs the four-threads-per-state form the Merkle builder
- * uses for narrow tree levels (Poseidon and Poseidon2 only). */
+ * cooperative != 0 (Poseidon and Poseidon2 only) runs another form: 2 and 3 the
+ * tensor-core one of the Merkle builder with 32 and 8 states per warp, other
+ * values the four-threads-per-state one of the device-resident loop. */
 RustError zeknox_permute(size_t device_id, uint64_t *states, uint64_t n, uint32_t hash_type, uint32_t cooperative,
                          void *stream);
 

@@ -1,0 +1,18 @@
+"""The tables of the tensor-core permutations (zeknox_b200/csrc/mma_tables.h):
+the permutations computed from them on the host, every byte-column sum as the
+tensor core takes it, equal the plain ones on corner and random states, and no
+sum reaches 2^24."""
+import os
+import subprocess
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def test_permutations_from_the_tables(tmp_path):
+    exe = tmp_path / "mma_perm"
+    r = subprocess.run(["g++", "-O2", "-std=c++17", os.path.join(ROOT, "tests", "c", "mma_perm.cpp"), "-o", str(exe)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+    assert r.stdout.split() == ["72", "states"]

@@ -15,8 +15,8 @@ the tuner checks that for each candidate against the default's output):
 * ``wide_level_nodes.<hash>`` (per log2 leaves): Merkle levels with at least this
   many nodes run one launch per level (one thread per node) before the
   in-CTA fold takes over;
-* ``coop_leaves.<hash>`` (per log2 leaves; Poseidon and Poseidon2): forests of at
-  most this many leaves hash their leaves with four threads per permutation;
+* ``coop_leaves.<hash>`` (per log2 leaves; Poseidon, Poseidon2 and Monolith):
+  forests of at most this many leaves hash them 8 per warp instead of 16 or 32;
 * ``ntt_split_logr`` (per log2 n): the largest pass, 2^7..2^10 points, of a
   column-output transform (compute_batched_ntt / compute_batched_lde); 0 keeps
   the built-in split;
@@ -43,21 +43,28 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.dirname(HERE))
 
-DEFAULTS = {"lde_last_logr": 8, "lde_chunk_mib": 512, "leaf_threads": 256, "wide_level_nodes": 1 << 15,
-            "coop_leaves": 1 << 13, "ntt_split_logr": 0, "transpose_bulk": 9}
+DEFAULTS = {"lde_last_logr": 8, "lde_chunk_mib": 512, "wide_level_nodes": 1 << 15, "coop_leaves": 1 << 12,
+            "ntt_split_logr": 0, "transpose_bulk": 9}
 CANDIDATES = {
     "lde_last_logr": [8, 7, 6],
     "lde_chunk_mib": [512, 96, 128, 256, 2048],
-    "leaf_threads": [256, 128, 64],
     "wide_level_nodes": [1 << 15, 1 << 13, 1 << 17, 1 << 40],
-    "coop_leaves": [1 << 13, 0, 1 << 40],
+    "coop_leaves": [1 << 12, 0, 1 << 40],
     "ntt_split_logr": [0, 10, 9, 8, 7],
     "transpose_bulk": [9, 0, 1, 3, 5],
 }
 SEARCHES = ("lde", "merkle", "ntt", "transpose")
-COOP_HASHES = (0, 3)  # hashes with the cooperative (four threads per permutation) kernels
+MMA_HASHES = (0, 3, 4)  # hashes whose linear layers run on the tensor cores, 8, 16 or 32 leaves per warp
 HASH_NAMES = {0: "poseidon", 1: "keccak", 3: "poseidon2", 4: "monolith"}
 RATE = 3
+
+
+def leaf_threads(h, lg):
+    """CTA sizes of the leaf kernel of hash h for 2^lg leaves, the built-in one first."""
+    if h not in MMA_HASHES:
+        return [256, 128, 64]
+    first = 32 if lg <= 15 else 128 if h == 4 else 64
+    return [first] + [t for t in (128, 64, 32) if t != first]
 
 
 def lde_shapes(quick):
@@ -186,11 +193,11 @@ def tune_merkle(zk, torch, timer, h, lg, leaf_size, margin, log):
             raise RuntimeError("%s forest 2^%d x %d differs with %s = %d" % (HASH_NAMES[h], lg, leaf_size, knob, v))
 
     print("Merkle %s 2^%d leaves x %d" % (HASH_NAMES[h], lg, leaf_size), flush=True)
-    search(zk, timer, "leaf_threads.%d" % h, lg, CANDIDATES["leaf_threads"], DEFAULTS["leaf_threads"], run, check,
-           margin, log)
+    threads = leaf_threads(h, lg)
+    search(zk, timer, "leaf_threads.%d" % h, lg, threads, threads[0], run, check, margin, log)
     search(zk, timer, "wide_level_nodes.%d" % h, lg, CANDIDATES["wide_level_nodes"], DEFAULTS["wide_level_nodes"],
            run, check, margin, log)
-    if h in COOP_HASHES:
+    if h in MMA_HASHES:
         search(zk, timer, "coop_leaves.%d" % h, lg, CANDIDATES["coop_leaves"], DEFAULTS["coop_leaves"], run, check,
                margin, log)
     del leaves, dig, caps, ref_d, ref_c

@@ -3,14 +3,13 @@
 // Follows native/merkle/merkle.cu:166-280 of zeknox for the layout and the
 // special cases (caps == leaves; subtrees of 1 or 2 leaves).  Launches: the
 // leaf kernel; one node-parallel level kernel per level while a level still
-// has >= wide_level_nodes nodes; the fold kernel (the next 8 levels inside
-// CTAs, and the caps when whole subtrees fit); for subtrees still above 1024
-// nodes, level kernels, then one tail CTA per subtree -- 2 to 6 launches where
-// the reference launches one per level.  Poseidon2's leaf kernel also builds
-// the first three levels above the leaves in its CTAs.  For Poseidon and Poseidon2 the fold
-// and tail kernels (and the leaf kernel of forests of at most coop_leaves
-// leaves) run one permutation per group of four threads (coop.cuh): the fold
-// kernel then takes 6 levels per launch.
+// has >= wide_level_nodes nodes; then folds inside CTAs.  Poseidon, Poseidon2
+// and Monolith run their linear layers on the tensor cores (hash_mma.cuh), 32,
+// 16 or 8 leaves per warp by the forest's size, and fold 6 levels per launch
+// until a CTA holds whole subtrees.  Keccak and Poseidon-BN128 hash one leaf
+// or node per thread: a fold kernel of 8 levels and, for subtrees still above
+// 1024 nodes, level kernels, then one tail CTA per subtree.
+#include <algorithm>
 #include <cstdio>
 #include <string>
 
@@ -21,14 +20,21 @@
 
 namespace zk {
 
-static constexpr int LEAF_T = 256;     // default leaves (threads) per CTA of the leaf kernel ("leaf_threads.<hash>")
-// Poseidon-BN128's leaf kernel holds 136 registers a thread: three 128-thread
-// CTAs fit an SM (12 warps) where one 256-thread CTA does (measured on 2^20 x
-// 135 forests: 450 against 491 ms; 2^14 x 135: 18.0 against 23.9 ms)
+// Default threads per CTA of the leaf kernel ("leaf_threads.<hash>", 32 for
+// the tensor-core hashes only).  Poseidon-BN128's holds 152 registers a
+// thread: three 128-thread CTAs fit an SM where one 256-thread CTA does.  The
+// tensor-core hashes take one-warp CTAs up to 2^15 leaves, where an SM has a
+// handful of warps and larger CTAs leave some SMs one more than others
+// (Poseidon2 2^15 x 135: 857 against 880 us with 64 threads, 837 at the
+// one-thread-per-leaf form; 2^14: 493 against 509), above that 64 (Poseidon2
+// 2^20 x 135: 14.11 against 14.18 ms) or, for Monolith, 128 (5.14 against 5.30).
+static constexpr int LEAF_T = 256;
 template <int H>
-constexpr int leaf_t_default()
+static uint64_t leaf_t_default(uint64_t n_leaves)
 {
-    return H == HASH_POSEIDON_BN128 ? 128 : LEAF_T;
+    if (H == HASH_POSEIDON_BN128) return 128;
+    if (!HasMma<H>::value) return LEAF_T;
+    return n_leaves <= (1ULL << 15) ? 32 : H == HASH_MONOLITH ? 128 : 64;
 }
 // Threads per CTA of the node-parallel level kernel: 128 for Poseidon-BN128
 // (158 registers: three CTAs per SM instead of one), 256 otherwise.  The wide
@@ -41,10 +47,19 @@ constexpr unsigned level_t()
 }
 static constexpr int FOLD_T = 256;     // leaf digests per CTA of the fold kernel
 static constexpr int TAIL_MAXM = 1024; // nodes a tail CTA can take
-static constexpr int LEAF_LEVELS = 3;  // tree levels the Poseidon2 leaf kernel folds in its CTAs
-static constexpr int COOP_T = 256;     // threads (64 groups of four) per CTA of the cooperative kernels
-static constexpr uint64_t COOP_LEAVES = 1ULL << 13;  // default: forests up to this many leaves hash their leaves
-                                                     // with the cooperative kernel ("coop_leaves.<hash>")
+// Leaves per warp of the tensor-core leaf kernel: 8 up to coop_leaves leaves
+// ("coop_leaves.<hash>"), 16 up to MID_LEAVES times as many, else 32.  Fewer
+// per warp are fewer S-boxes in sequence and more warps, for more instructions
+// a leaf.  Measured on B200, forests of 135-word leaves, 8 / 16 / 32 per warp
+// (us): Poseidon 2^12 353 / 413 / 710, 2^14 652 / 499 / 708, 2^15 978 / 939 /
+// 857; Poseidon2 the same within 5%; Monolith 2^12 108 / 128 / 214, 2^16
+// 433 / 374 / 454, 2^17 800 / 679 / 740.
+static constexpr uint64_t COOP_LEAVES = 1ULL << 12;
+template <int H>
+constexpr uint64_t mid_leaves()
+{
+    return H == HASH_MONOLITH ? 32 : 4;
+}
 static constexpr uint64_t WIDE_LEVEL_NODES = 1ULL << 15;  // default: levels at least this wide run node-parallel
                                                           // ("wide_level_nodes.<hash>")
 
@@ -53,40 +68,63 @@ bool merkle_geometry_ok(uint64_t n_digests, uint64_t n_caps, uint64_t n_leaves, 
     return merkle_geometry_check(n_digests, n_caps, n_leaves, cap_height, err);
 }
 
+template <int H, int NS, int T>
+static void launch_leaf_mma_t(uint64_t *digests, uint64_t *caps, const uint64_t *leaves, const MerkleGeom &g, cudaStream_t s)
+{
+    constexpr uint64_t per = (uint64_t)(T / 32) * 8 * NS;
+    merkle_leaf_mma_kernel<H, NS, T><<<(unsigned)((g.n_leaves + per - 1) / per), T, 0, s>>>(leaves, digests, caps, g);
+}
+
+template <int H, int NS>
+static void launch_leaf_mma(uint64_t lt, uint64_t *digests, uint64_t *caps, const uint64_t *leaves, const MerkleGeom &g,
+                            cudaStream_t s)
+{
+    if (lt == 32) launch_leaf_mma_t<H, NS, 32>(digests, caps, leaves, g, s);
+    else if (lt == 64) launch_leaf_mma_t<H, NS, 64>(digests, caps, leaves, g, s);
+    else launch_leaf_mma_t<H, NS, 128>(digests, caps, leaves, g, s);
+}
+
+// One level, one node per thread, or 32 per warp.
+template <int H>
+static void launch_level(uint64_t total, uint64_t *digests, const MerkleGeom &g, uint32_t u, cudaStream_t s)
+{
+    if constexpr (HasMma<H>::value) {
+        merkle_level_mma_kernel<H, 4, 128><<<(unsigned)((total + 127) / 128), 128, 0, s>>>(digests, g, u);
+    } else {
+        uint64_t nb = (total + level_t<H>() - 1) / level_t<H>();
+        if (nb > 65535) nb = 65535;
+        merkle_level_kernel<H><<<(unsigned)nb, level_t<H>(), 0, s>>>(digests, g, u);
+    }
+    note_launch();
+}
+
 template <int H>
 static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *leaves, const MerkleGeom &g, cudaStream_t s)
 {
-    constexpr bool COOP = HasCoop<H>::value;
     const uint32_t lg_leaves = ilog2_exact(g.n_leaves);
-    const uint64_t lt = tune_get("leaf_threads." + std::to_string(H), lg_leaves, leaf_t_default<H>());
+    const uint64_t lt = tune_get("leaf_threads." + std::to_string(H), lg_leaves, leaf_t_default<H>(g.n_leaves));
     uint64_t blocks;
-    bool coop_leaf = false;
-    if constexpr (COOP) coop_leaf = g.n_leaves <= tune_get("coop_leaves." + std::to_string(H), lg_leaves, COOP_LEAVES);
+    uint64_t coop = 0;
+    if constexpr (HasMma<H>::value)
+        coop = std::min<uint64_t>(tune_get("coop_leaves." + std::to_string(H), lg_leaves, COOP_LEAVES), 1ULL << 40);
     uint32_t u0 = 0;
-    // Poseidon2: the first LEAF_LEVELS tree levels inside the leaf kernel's
-    // CTAs (measured 1.006x on Poseidon2 forests, 0.97x on Poseidon's)
-    const bool fused = H == HASH_POSEIDON2 && !coop_leaf && lt == (uint64_t)LEAF_T &&
-                       g.sub_leaves >= (uint64_t)LEAF_T && g.log_sub > (uint32_t)LEAF_LEVELS;
-    if (fused) {
-        if constexpr (H == HASH_POSEIDON2) {
-            blocks = g.n_leaves / LEAF_T;
-            merkle_leaf_levels_kernel<H, LEAF_T, LEAF_LEVELS><<<(unsigned)blocks, LEAF_T, 0, s>>>(leaves, digests, g);
-            u0 = LEAF_LEVELS;
-        }
-    } else if (coop_leaf) {
-        if constexpr (COOP) {
-            blocks = (g.n_leaves + COOP_T / 4 - 1) / (COOP_T / 4);
-            merkle_leaf_coop_kernel<H, COOP_T><<<(unsigned)blocks, COOP_T, 0, s>>>(leaves, digests, caps, g);
+    bool mma_leaf = false;
+    if constexpr (HasMma<H>::value) mma_leaf = g.leaf_size > 4;
+    if (mma_leaf) {
+        if constexpr (HasMma<H>::value) {
+            if (g.n_leaves <= coop) launch_leaf_mma<H, 1>(lt, digests, caps, leaves, g, s);
+            else if (g.n_leaves <= mid_leaves<H>() * coop) launch_leaf_mma<H, 2>(lt, digests, caps, leaves, g, s);
+            else launch_leaf_mma<H, 4>(lt, digests, caps, leaves, g, s);
         }
     } else if (lt == 64) {
         blocks = (g.n_leaves + 63) / 64;
-        merkle_leaf_kernel_for<H, 64>()<<<(unsigned)blocks, 64, 0, s>>>(leaves, digests, caps, g);
+        merkle_leaf_kernel<H, 64><<<(unsigned)blocks, 64, 0, s>>>(leaves, digests, caps, g);
     } else if (lt == 128) {
         blocks = (g.n_leaves + 127) / 128;
-        merkle_leaf_kernel_for<H, 128>()<<<(unsigned)blocks, 128, 0, s>>>(leaves, digests, caps, g);
+        merkle_leaf_kernel<H, 128><<<(unsigned)blocks, 128, 0, s>>>(leaves, digests, caps, g);
     } else {
         blocks = (g.n_leaves + LEAF_T - 1) / LEAF_T;
-        merkle_leaf_kernel_for<H, LEAF_T>()<<<(unsigned)blocks, LEAF_T, 0, s>>>(leaves, digests, caps, g);
+        merkle_leaf_kernel<H, LEAF_T><<<(unsigned)blocks, LEAF_T, 0, s>>>(leaves, digests, caps, g);
     }
     note_launch();
     const uint64_t wide = tune_get("wide_level_nodes." + std::to_string(H), lg_leaves, WIDE_LEVEL_NODES);
@@ -96,34 +134,36 @@ static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *lea
     while (u0 + 1 <= top && (g.n_leaves >> (u0 + 1)) >= wide) {
         u0++;
         const uint64_t total = g.n_leaves >> u0;
-        merkle_level_kernel<H><<<(unsigned)((total + level_t<H>() - 1) / level_t<H>()), level_t<H>(), 0, s>>>(digests, g,
-                                                                                                          u0);
+        launch_level<H>(total, digests, g, u0, s);
+    }
+    // Narrow levels: folded inside CTAs of fold_nodes nodes; the tensor-core
+    // form repeats until its CTAs hold whole subtrees.
+    if constexpr (HasMma<H>::value) {
+        for (;;) {
+            const uint64_t count = g.n_leaves >> u0;
+            merkle_fold_mma_kernel<H><<<(unsigned)((count + MMA_FOLD_IN - 1) / MMA_FOLD_IN), 128, 0, s>>>(digests, caps, g, u0);
+            note_launch();
+            if ((g.sub_leaves >> u0) <= MMA_FOLD_IN) return;  // caps written
+            u0 += __builtin_ctz(MMA_FOLD_IN);
+        }
+    } else {
+        const uint64_t count = g.n_leaves >> u0;
+        blocks = (count + FOLD_T - 1) / FOLD_T;
+        merkle_fold_kernel<H, FOLD_T><<<(unsigned)blocks, FOLD_T, 0, s>>>(digests, caps, g, u0);
+        note_launch();
+        const uint64_t sub_nodes = g.sub_leaves >> u0;
+        if (sub_nodes <= (uint64_t)FOLD_T) return;  // caps written by the fold kernel
+        // heights folded by the fold kernel
+        uint32_t U = 0;
+        while ((1u << (U + 1)) <= FOLD_T && u0 + U + 1 <= top) U++;
+        u0 += U;
+        while ((g.sub_leaves >> u0) > (uint64_t)TAIL_MAXM) {
+            u0++;
+            launch_level<H>((g.sub_leaves >> u0) * g.n_caps, digests, g, u0, s);
+        }
+        merkle_tail_kernel<H, TAIL_MAXM><<<g.n_caps, 256, 0, s>>>(digests, caps, g, u0);
         note_launch();
     }
-    // Narrow levels: folded inside CTAs of fold_nodes nodes.
-    const uint32_t fold_nodes = COOP ? COOP_T / 4 : FOLD_T;
-    const uint64_t count = g.n_leaves >> u0;
-    blocks = (count + fold_nodes - 1) / fold_nodes;
-    if constexpr (COOP) merkle_fold_coop_kernel<H, COOP_T><<<(unsigned)blocks, COOP_T, 0, s>>>(digests, caps, g, u0);
-    else merkle_fold_kernel<H, FOLD_T><<<(unsigned)blocks, FOLD_T, 0, s>>>(digests, caps, g, u0);
-    note_launch();
-    const uint64_t sub_nodes = g.sub_leaves >> u0;
-    if (sub_nodes <= (uint64_t)fold_nodes) return;  // caps written by the fold kernel
-    // heights folded by the fold kernel
-    uint32_t U = 0;
-    while ((1u << (U + 1)) <= fold_nodes && u0 + U + 1 <= top) U++;
-    u0 += U;
-    while ((g.sub_leaves >> u0) > (uint64_t)TAIL_MAXM) {
-        u0++;
-        uint64_t total = (g.sub_leaves >> u0) * g.n_caps;
-        uint64_t nb = (total + level_t<H>() - 1) / level_t<H>();
-        if (nb > 65535) nb = 65535;
-        merkle_level_kernel<H><<<(unsigned)nb, level_t<H>(), 0, s>>>(digests, g, u0);
-        note_launch();
-    }
-    if constexpr (COOP) merkle_tail_coop_kernel<H, TAIL_MAXM><<<g.n_caps, 256, 0, s>>>(digests, caps, g, u0);
-    else merkle_tail_kernel<H, TAIL_MAXM><<<g.n_caps, 256, 0, s>>>(digests, caps, g, u0);
-    note_launch();
 }
 
 bool merkle_device(uint64_t *digests, uint64_t *caps, const uint64_t *leaves, uint64_t n_digests, uint64_t n_caps,

@@ -9,7 +9,8 @@
 //
 // Kernel structure (B200-first instead of one launch per level):
 //   * leaf kernel: one thread per leaf runs the sponge with the state in
-//     registers (nothing else, so no warp idles on a barrier);
+//     registers (nothing else, so no warp idles on a barrier), or a warp 8, 16
+//     or 32 leaves with the linear layers on the tensor cores;
 //   * level kernel: one thread per node of one level, for the wide levels
 //     just above the leaves (and for levels a tail CTA cannot hold);
 //   * fold kernel: each CTA folds T consecutive nodes log2(T) levels up in
@@ -20,8 +21,8 @@
 #include <stdint.h>
 
 #include "bounds.cuh"
-#include "coop.cuh"
 #include "hash.cuh"
+#include "hash_mma.cuh"
 
 namespace zk {
 
@@ -86,61 +87,6 @@ __global__ void __launch_bounds__(T)
                        MerkleGeom g)
 {
     merkle_leaf_body<H, T>(leaves, digests, caps, g);
-}
-
-// The same, held to 1024 threads per SM (64 registers): measured 1.02-1.03x
-// for Poseidon and Poseidon2 leaves on B200, and slower for the other hashes,
-// which keep the unconstrained kernel above.
-template <int H, int T>
-__global__ void __launch_bounds__(T, 1024 / T)
-    merkle_leaf_kernel_1k(const uint64_t *__restrict__ leaves, uint64_t *__restrict__ digests,
-                          uint64_t *__restrict__ caps, MerkleGeom g)
-{
-    merkle_leaf_body<H, T>(leaves, digests, caps, g);
-}
-
-// Leaf digests plus the LV tree levels above them inside the CTA (sponge
-// hashes only; needs T leaves per CTA inside one subtree and LV < log2 T,
-// LV <= the subtree's top height).  A node is the sponge hash of its two
-// children's 8 consecutive words, so leaves and nodes go through the same
-// call site and the permutation's code exists once.
-template <int H, int T, int LV>
-__global__ void __launch_bounds__(T, 1024 / T)
-    merkle_leaf_levels_kernel(const uint64_t *__restrict__ leaves, uint64_t *__restrict__ digests, MerkleGeom g)
-{
-    __shared__ uint64_t nd[T][4];
-    const uint64_t i0 = (uint64_t)blockIdx.x * T;
-    const uint32_t t = threadIdx.x;
-#pragma unroll 1
-    for (int v = 0; v <= LV; v++) {
-        const uint32_t nodes = T >> v;
-        uint64_t h[4];
-        if (t < nodes) {
-            const uint64_t *src = v == 0 ? leaves + (i0 + t) * g.leaf_size : &nd[2 * t][0];
-            const bool row_ok =
-                v != 0 || ZK_IN_BOUNDS((i0 + t + 1) * g.leaf_size - 1, merkle_leaf_words(g), OOB_MERKLE_LEAF);
-            if (row_ok) sponge_hash_one<H>(src, v == 0 ? g.leaf_size : 8, h);
-            const uint64_t di = merkle_node_index(g, i0 + ((uint64_t)t << v), (uint32_t)v);
-            if (row_ok && ZK_IN_BOUNDS(4 * di + 3, merkle_digest_words(g), OOB_MERKLE_DIGEST)) {
-#pragma unroll
-                for (int q = 0; q < 4; q++) digests[4 * di + q] = h[q];
-            }
-        }
-        __syncthreads();
-        if (t < nodes) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) nd[t][q] = h[q];
-        }
-        __syncthreads();
-    }
-}
-
-// Leaf kernel of hash H with CTAs of T threads.
-template <int H, int T>
-constexpr auto merkle_leaf_kernel_for()
-{
-    if constexpr (H == HASH_POSEIDON || H == HASH_POSEIDON2) return merkle_leaf_kernel_1k<H, T>;
-    else return merkle_leaf_kernel<H, T>;
 }
 
 // Folds stored digests upwards from height u0 (0 = leaf digests): each CTA
@@ -271,158 +217,125 @@ __global__ void merkle_level_kernel(uint64_t *__restrict__ digests, MerkleGeom g
     }
 }
 
-// ------------------------------------------------------ cooperative kernels
+// ------------------------------------------------------ tensor-core kernels
 //
-// Poseidon and Poseidon2 with one permutation per group of four threads
-// (coop.cuh): the leaves of forests too small to fill the GPU with one leaf
-// per thread, and the tree levels below the wide ones, whose time is the
-// latency of one permutation per level.  A warp holds eight groups; a group
-// with nothing to do hashes a copy of its warp's first task and writes
-// nothing, and a warp with nothing to do skips the level, so the full-warp
-// shuffles always see all 32 threads.
+// Poseidon and Poseidon2 with the linear layers on the tensor cores
+// (hash_mma.cuh): a warp hashes 8 * NS leaves or nodes, row q * 8 + g of its
+// span being state q of quad g.  Rows past the end repeat the last one and
+// store nothing.
 
-// Leaf digests, one leaf per group.
-template <int H, int T>
-__global__ void __launch_bounds__(T)
-    merkle_leaf_coop_kernel(const uint64_t *__restrict__ leaves, uint64_t *__restrict__ digests,
-                            uint64_t *__restrict__ caps, MerkleGeom g)
+// Threads per SM the register budget of the 32-leaf form aims at: 640 (96
+// registers).  Poseidon2 2^20 x 135: 14.26 ms against 14.44 at 512; 768 and
+// 1024 spill and were slower (an earlier form: 15.2 and 19.8 against 14.9).
+static constexpr int MMA_THREADS_PER_SM = 640;
+
+// Leaf digests (leaf_size > 4: shorter leaves are copied, not hashed).
+template <int H, int NS, int T>
+__global__ void __launch_bounds__(T, NS == 4 ? MMA_THREADS_PER_SM / T : 1)
+    merkle_leaf_mma_kernel(const uint64_t *__restrict__ leaves, uint64_t *__restrict__ digests,
+                           uint64_t *__restrict__ caps, MerkleGeom g)
 {
-    CoopGroup c;
-    c.init();
-    const uint64_t gi = ((uint64_t)blockIdx.x * T + threadIdx.x) >> 2;
-    if ((gi & ~7ULL) >= g.n_leaves) return;  // the whole warp is past the end
-    const uint64_t i = gi < g.n_leaves ? gi : g.n_leaves - 1;
-    uint64_t d[4];
-    // (every thread of the warp runs the permutation: a row out of range is
-    // hashed from row 0 and its digest not written)
-    const bool row_ok = !g.leaf_size || ZK_IN_BOUNDS((i + 1) * g.leaf_size - 1, merkle_leaf_words(g), OOB_MERKLE_LEAF);
-    sponge_hash_one_coop<H>(leaves + (row_ok ? i : 0) * g.leaf_size, g.leaf_size, d, c);
-    const bool dst_ok = g.sub_leaves == 1
-                            ? ZK_IN_BOUNDS(4 * gi + 3, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)
-                            : ZK_IN_BOUNDS(4 * merkle_node_index(g, gi, 0) + 3, merkle_digest_words(g), OOB_MERKLE_DIGEST);
-    if (c.q == 0 && gi < g.n_leaves && row_ok && dst_ok) {
-        uint64_t *dst = g.sub_leaves == 1 ? caps + 4 * gi : digests + 4 * merkle_node_index(g, gi, 0);
+    __shared__ __align__(16) uint32_t sm[T / 32][MmaSmem<NS>::template words<H>()];
+    const uint32_t warp = threadIdx.x >> 5, quad = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const uint64_t first = ((uint64_t)blockIdx.x * (T / 32) + warp) * (8 * NS) + quad;
+    if (first - quad >= g.n_leaves) return;  // the whole warp is past the end
+    uint64_t d[NS];
+    auto row = [&](int q) {
+        const uint64_t i = first + 8 * q < g.n_leaves ? first + 8 * q : g.n_leaves - 1;
+        return leaves + (ZK_IN_BOUNDS((i + 1) * g.leaf_size - 1, merkle_leaf_words(g), OOB_MERKLE_LEAF) ? i : 0) * g.leaf_size;
+    };
+    sponge_hash_mma<H, NS>(row, g.leaf_size, sm[warp], d);
 #pragma unroll
-        for (int q = 0; q < 4; q++) dst[q] = d[q];
+    for (int q = 0; q < NS; q++) {
+        const uint64_t i = first + 8 * q;
+        if (i >= g.n_leaves) continue;
+        // caps == leaves: the leaf hashes are the caps
+        if (g.sub_leaves == 1) {
+            if (ZK_IN_BOUNDS(4 * i + t, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)) caps[4 * i + t] = d[q];
+        } else {
+            const uint64_t w = 4 * merkle_node_index(g, i, 0) + t;
+            if (ZK_IN_BOUNDS(w, merkle_digest_words(g), OOB_MERKLE_DIGEST)) digests[w] = d[q];
+        }
     }
 }
 
-// merkle_fold_kernel with T / 4 nodes of height u0 per CTA.
-template <int H, int T>
-__global__ void __launch_bounds__(T) merkle_fold_coop_kernel(uint64_t *__restrict__ digests, uint64_t *__restrict__ caps,
-                                                             MerkleGeom g, uint32_t u0)
+// One level of height u, every node of every subtree.
+template <int H, int NS, int T>
+__global__ void __launch_bounds__(T, NS == 4 ? MMA_THREADS_PER_SM / T : 1)
+    merkle_level_mma_kernel(uint64_t *__restrict__ digests, MerkleGeom g, uint32_t u)
 {
-    constexpr uint32_t NG = T / 4;
-    __shared__ uint64_t node[NG][4];
-    CoopGroup c;
-    c.init();
-    const uint32_t grp = threadIdx.x >> 2;
-    const uint32_t wg = grp & ~7u;  // first group of this warp
+    __shared__ __align__(16) uint32_t sm[T / 32][MmaSmem<NS>::template words<H>()];
+    const uint32_t warp = threadIdx.x >> 5, quad = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const uint64_t total = g.n_leaves >> u;
+    const uint64_t first = ((uint64_t)blockIdx.x * (T / 32) + warp) * (8 * NS) + quad;
+    if (first - quad >= total) return;
+    uint64_t d[NS];
+    auto row = [&](int q) {
+        const uint64_t x = first + 8 * q < total ? first + 8 * q : total - 1;
+        // the two children of a node are neighbours: eight consecutive words
+        const uint64_t w = 4 * merkle_node_index(g, x << u, u - 1);
+        return (const uint64_t *)digests + (ZK_IN_BOUNDS(w + 7, merkle_digest_words(g), OOB_MERKLE_NODE) ? w : 0);
+    };
+    sponge_hash_mma<H, NS>(row, 8, sm[warp], d);
+#pragma unroll
+    for (int q = 0; q < NS; q++) {
+        const uint64_t x = first + 8 * q;
+        if (x >= total) continue;
+        const uint64_t w = 4 * merkle_node_index(g, x << u, u) + t;
+        if (ZK_IN_BOUNDS(w, merkle_digest_words(g), OOB_MERKLE_DIGEST)) digests[w] = d[q];
+    }
+}
+
+// merkle_fold_kernel for the tensor-core hashes: a CTA of four warps takes
+// MMA_FOLD_IN consecutive nodes of height u0 (its first level is one
+// permutation per quad of threads) and computes every node above them whose
+// subtree lies in the CTA, and the caps of subtrees that fit.  What these
+// narrow levels wait on is the latency of one permutation per level: 8 states
+// per warp (NS = 1), a third of the lanes' S-boxes per thread.
+static constexpr uint32_t MMA_FOLD_IN = 64;
+
+template <int H>
+__global__ void __launch_bounds__(128) merkle_fold_mma_kernel(uint64_t *__restrict__ digests, uint64_t *__restrict__ caps,
+                                                              MerkleGeom g, uint32_t u0)
+{
+    __shared__ __align__(16) uint32_t sm[4][MmaSmem<1>::words<H>()];
+    __shared__ uint64_t node[MMA_FOLD_IN][4];
+    const uint32_t quad = threadIdx.x >> 2, t = threadIdx.x & 3, warp = threadIdx.x >> 5;
+    const uint32_t wq = quad & ~7u;  // first quad of this warp
     const uint64_t count = g.n_leaves >> u0;
-    const uint64_t i0 = (uint64_t)blockIdx.x * NG;
-    const uint64_t cta_nodes = count - i0 < (uint64_t)NG ? count - i0 : (uint64_t)NG;
-    for (uint32_t t = threadIdx.x; t < 4 * cta_nodes; t += T) {
-        const uint64_t wi = 4 * merkle_node_index(g, (i0 + (t >> 2)) << u0, u0) + (t & 3);
-        node[t >> 2][t & 3] = ZK_IN_BOUNDS(wi, merkle_digest_words(g), OOB_MERKLE_NODE) ? digests[wi] : 0;
+    const uint64_t i0 = (uint64_t)blockIdx.x * MMA_FOLD_IN;
+    const uint64_t cta_nodes = count - i0 < MMA_FOLD_IN ? count - i0 : MMA_FOLD_IN;
+    for (uint32_t k = threadIdx.x; k < 4 * cta_nodes; k += 128) {
+        const uint64_t wi = 4 * merkle_node_index(g, (i0 + (k >> 2)) << u0, u0) + (k & 3);
+        node[k >> 2][k & 3] = ZK_IN_BOUNDS(wi, merkle_digest_words(g), OOB_MERKLE_NODE) ? digests[wi] : 0;
     }
     const uint32_t top = g.log_sub - 1;
     uint32_t U = 0;
-    while ((1u << (U + 1)) <= NG && u0 + U + 1 <= top) U++;
-    for (uint32_t v = 1; v <= U; v++) {
-        __syncthreads();
-        const uint32_t nodes = NG >> v;
-        const bool act = grp < nodes && ((uint64_t)grp << v) < cta_nodes;
-        const bool wact = wg < nodes && ((uint64_t)wg << v) < cta_nodes;
-        uint64_t h[4];
-        if (wact) {
-            const uint32_t src = act ? grp : wg;
-            sponge_hash_two_coop<H>(node[2 * src], node[2 * src + 1], h, c);
-            if (act && c.q == 0) {
-                const uint64_t di = merkle_node_index(g, (i0 + ((uint64_t)grp << v)) << u0, u0 + v);
-                if (ZK_IN_BOUNDS(4 * di + 3, merkle_digest_words(g), OOB_MERKLE_DIGEST)) {
-#pragma unroll
-                    for (int q = 0; q < 4; q++) digests[4 * di + q] = h[q];
-                }
-            }
-        }
-        __syncthreads();
-        if (act && c.q == 0) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) node[grp][q] = h[q];
-        }
-    }
+    while ((1u << (U + 1)) <= MMA_FOLD_IN && u0 + U + 1 <= top) U++;
     const uint64_t sub_nodes = g.sub_leaves >> u0;
-    if (u0 + U == top && sub_nodes <= (uint64_t)NG) {
+    // levels 1..U, then the caps when whole subtrees fit in the CTA
+    const uint32_t last = u0 + U == top && sub_nodes <= MMA_FOLD_IN ? U + 1 : U;
+#pragma unroll 1
+    for (uint32_t v = 1; v <= last; v++) {
         __syncthreads();
-        const uint32_t subs = (uint32_t)(cta_nodes / sub_nodes);
-        if (wg < subs) {
-            const bool act = grp < subs;
-            const uint32_t src = act ? grp : wg;
-            uint64_t h[4];
-            sponge_hash_two_coop<H>(node[2 * src], node[2 * src + 1], h, c);
-            if (act && c.q == 0) {
-                const uint64_t k = ((i0 << u0) >> g.log_sub) + grp;
-                if (ZK_IN_BOUNDS(4 * k + 3, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)) {
-#pragma unroll
-                    for (int q = 0; q < 4; q++) caps[4 * k + q] = h[q];
-                }
+        // nodes of this level in the CTA (at the caps: its subtrees)
+        const uint32_t nodes = v <= U ? (uint32_t)((cta_nodes + (1u << v) - 1) >> v) : (uint32_t)(cta_nodes / sub_nodes);
+        const bool act = quad < nodes;
+        uint64_t h[1];
+        if (wq < nodes) {
+            // a quad with no node repeats its warp's first
+            const uint64_t *src = &node[2 * (act ? quad : wq)][0];
+            sponge_hash_mma<H, 1>([&](int) { return src; }, 8, sm[warp], h);
+            if (act && v <= U) {
+                const uint64_t w = 4 * merkle_node_index(g, (i0 + ((uint64_t)quad << v)) << u0, u0 + v) + t;
+                if (ZK_IN_BOUNDS(w, merkle_digest_words(g), OOB_MERKLE_DIGEST)) digests[w] = h[0];
+            } else if (act) {
+                const uint64_t w = 4 * (((i0 << u0) >> g.log_sub) + quad) + t;
+                if (ZK_IN_BOUNDS(w, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)) caps[w] = h[0];
             }
         }
-    }
-}
-
-// merkle_tail_kernel with one permutation per group: one CTA of 256 threads
-// (64 groups) per subtree.
-template <int H, int MAXM>
-__global__ void __launch_bounds__(256) merkle_tail_coop_kernel(uint64_t *__restrict__ digests, uint64_t *__restrict__ caps,
-                                                               MerkleGeom g, uint32_t u0)
-{
-    constexpr uint32_t NG = 256 / 4;
-    __shared__ uint64_t bufa[MAXM][4];
-    __shared__ uint64_t bufb[MAXM / 2][4];
-    CoopGroup c;
-    c.init();
-    const uint32_t grp = threadIdx.x >> 2;
-    const uint64_t k = blockIdx.x;
-    uint64_t *sub = digests + k * g.sub_digests * 4;
-    const uint64_t sub0 = k * g.sub_digests * 4;
-    uint32_t m = (uint32_t)(g.sub_leaves >> u0);
-    for (uint32_t j = threadIdx.x; j < 4 * m; j += 256)
-        bufa[j >> 2][j & 3] =
-            ZK_IN_BOUNDS(sub0 + 4 * (m - 2) + j, merkle_digest_words(g), OOB_MERKLE_NODE) ? sub[4 * (m - 2) + j] : 0;
-    uint64_t(*src)[4] = bufa;
-    uint64_t(*dst)[4] = bufb;
-    while (m > 2) {
         __syncthreads();
-        const uint32_t half = m / 2;
-        for (uint32_t base = grp & ~7u; base < half; base += NG) {
-            const uint32_t j = base + (grp & 7u);
-            const bool act = j < half;
-            const uint32_t jj = act ? j : base;
-            uint64_t h[4];
-            sponge_hash_two_coop<H>(src[2 * jj], src[2 * jj + 1], h, c);
-            if (act && c.q == 0) {
-                const bool ok = ZK_IN_BOUNDS(sub0 + 4 * (half - 2 + j) + 3, merkle_digest_words(g), OOB_MERKLE_DIGEST);
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    if (ok) sub[4 * (half - 2 + j) + q] = h[q];
-                    dst[j][q] = h[q];
-                }
-            }
-        }
-        uint64_t(*tmp)[4] = src;
-        src = dst;
-        dst = tmp;
-        m = half;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        uint64_t h[4];
-        sponge_hash_two_coop<H>(src[0], src[1], h, c);
-        if (threadIdx.x == 0 && ZK_IN_BOUNDS(4 * k + 3, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) caps[4 * k + q] = h[q];
-        }
+        if (act && v <= U) node[quad][t] = h[0];
     }
 }
 

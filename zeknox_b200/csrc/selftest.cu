@@ -19,6 +19,7 @@
 #include "coop.cuh"
 #include "gl64.cuh"
 #include "hash.cuh"
+#include "hash_mma.cuh"
 #include "ntt.cuh"
 #include "runtime.cuh"
 
@@ -156,6 +157,34 @@ __global__ void permute_coop_kernel(uint64_t *states, uint64_t n)
     }
 }
 
+// The tensor-core form of hash_mma.cuh, 8 * NS states per warp; states past n
+// are zero and not stored.
+template <int H, int NS>
+__global__ void __launch_bounds__(128) permute_mma_kernel(uint64_t *states, uint64_t n)
+{
+    __shared__ __align__(16) uint32_t sm[4][MmaSmem<NS>::WORDS];
+    const uint32_t warp = threadIdx.x >> 5, quad = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const uint64_t first = ((uint64_t)blockIdx.x * 4 + warp) * (8 * NS) + quad;
+#pragma unroll
+    for (int kb = 0; kb < 3; kb++)
+#pragma unroll
+        for (int q = 0; q < NS; q++)
+            mma_set_lane<NS>(sm[warp], kb, q, first + 8 * q < n ? states[(first + 8 * q) * 12 + 4 * kb + t] : 0);
+    permute_mma<H, NS>(sm[warp], 7u);
+#pragma unroll
+    for (int kb = 0; kb < 3; kb++)
+#pragma unroll
+        for (int q = 0; q < NS; q++)
+            if (first + 8 * q < n) states[(first + 8 * q) * 12 + 4 * kb + t] = gl_canon(mma_lane<NS>(sm[warp], kb, q));
+}
+
+template <int H>
+void launch_permute_mma(uint64_t *states, uint64_t n, bool wide, cudaStream_t s)
+{
+    if (wide) permute_mma_kernel<H, 4><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(states, n);
+    else permute_mma_kernel<H, 1><<<(unsigned)((n + 31) / 32), 128, 0, s>>>(states, n);
+}
+
 void check_launch(const char *what)
 {
     const cudaError_t e = cudaGetLastError();
@@ -204,7 +233,10 @@ extern "C" RustError zeknox_permute(size_t device_id, uint64_t *states, uint64_t
         if (n) {
             const uint64_t threads = cooperative ? 4 * n : n;
             const unsigned blocks = (unsigned)((threads + 127) / 128);
-            if (cooperative) {
+            if (cooperative == 2 || cooperative == 3) {
+                if (hash_type == HASH_POSEIDON) launch_permute_mma<HASH_POSEIDON>(states, n, cooperative == 2, s);
+                else launch_permute_mma<HASH_POSEIDON2>(states, n, cooperative == 2, s);
+            } else if (cooperative) {
                 if (hash_type == HASH_POSEIDON) permute_coop_kernel<HASH_POSEIDON><<<blocks, 128, 0, s>>>(states, n);
                 else permute_coop_kernel<HASH_POSEIDON2><<<blocks, 128, 0, s>>>(states, n);
             } else {
