@@ -455,6 +455,9 @@ ZK_HD void keccak_f(uint64_t st[25])
 // built with different settings hold different bodies of the functions
 // below; they are force-inlined (no out-of-line host symbol), the steps they
 // call are file-local, and device code is not linked across units.
+#ifndef ZK_BN128_LIMBS29
+#define ZK_BN128_LIMBS29 0
+#endif
 #ifndef ZK_BN128_DOT_ONE_REDUCTION
 #define ZK_BN128_DOT_ONE_REDUCTION 1
 #endif
@@ -565,6 +568,15 @@ ZK_HD void poseidon_bn128_permute(uint64_t s[12])
     }
 }
 
+// Units that define ZK_BN128_LIMBS29 run the device permutation on 29-bit limbs
+// (bn254_29.cuh); the device-resident request loop, whose stages share a
+// 64-register budget, does not.
+#if defined(__CUDACC__) && ZK_BN128_LIMBS29
+}  // namespace zk
+#include "bn254_29.cuh"
+namespace zk {
+#endif
+
 // ------------------------------------------------------------------ sponges
 
 template <int H>
@@ -572,7 +584,13 @@ ZK_HD void permute(uint64_t s[12])
 {
     if (H == HASH_POSEIDON) poseidon_permute(s);
     else if (H == HASH_POSEIDON2) poseidon2_permute(s);
-    else if (H == HASH_POSEIDON_BN128) poseidon_bn128_permute(s);
+    else if (H == HASH_POSEIDON_BN128) {
+#if defined(__CUDA_ARCH__) && ZK_BN128_LIMBS29
+        poseidon_bn128_permute29(s);
+#else
+        poseidon_bn128_permute(s);
+#endif
+    }
     else monolith_permute(s);
 }
 

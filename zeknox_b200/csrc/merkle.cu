@@ -9,6 +9,7 @@
 // until a CTA holds whole subtrees.  Keccak and Poseidon-BN128 hash one leaf
 // or node per thread: a fold kernel of 8 levels and, for subtrees still above
 // 1024 nodes, level kernels, then one tail CTA per subtree.
+#define ZK_BN128_LIMBS29 1
 #include <algorithm>
 #include <cstdio>
 #include <string>

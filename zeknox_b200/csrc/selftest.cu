@@ -9,6 +9,7 @@
 // compare with exact arithmetic, and run whole permutations on chosen states.
 // No reference counterpart (the reference's tests call its primitives from a
 // test binary, native/tests/tests.cu).
+#define ZK_BN128_LIMBS29 1
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
