@@ -643,7 +643,7 @@ void prepare_tables(DeviceCtx &c, uint32_t lg_n, uint32_t rate, uint64_t coset_g
 
 // The bulk-copy transpose: persistent CTAs, as many as fit on the SMs with
 // their stage buffers.
-template <uint32_t TI, uint32_t TB, uint32_t ST>
+template <uint32_t TI, uint32_t TB, uint32_t ST, int VEC = 2>
 static void launch_transpose_bulk(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint32_t lg, uint64_t cols,
                                   uint32_t extra, uint64_t wait_ns)
 {
@@ -651,17 +651,33 @@ static void launch_transpose_bulk(DeviceCtx &c, uint64_t *out, const uint64_t *i
     static int per_sm_of[64] = {};  // per device, set once under its lock
     int &per_sm = per_sm_of[c.id & 63];
     if (!per_sm) {
-        ZK_CUDA(cudaFuncSetAttribute(transpose_rev_bulk_kernel<TI, TB, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        ZK_CUDA(cudaFuncSetAttribute(transpose_rev_bulk_kernel<TI, TB, ST, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)G::SMEM_BYTES));
-        ZK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, transpose_rev_bulk_kernel<TI, TB, ST>, G::THREADS,
+        ZK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, transpose_rev_bulk_kernel<TI, TB, ST, VEC>, G::THREADS,
                                                               G::SMEM_BYTES));
         if (per_sm < 1) per_sm = 1;
     }
     const uint64_t n = 1ULL << lg;
-    const uint64_t tiles_i = n / TI, n_tiles = tiles_i * ((cols + TB - 1) / TB);
+    // 8-byte stores: the columns dealt out evenly over the fewest tiles (2^18 x
+    // 85 90 against 113 us, x 33 47 against 54); 16-byte ones keep rows of whole
+    // 512-byte runs (x 136 135 against 157 us dealt out evenly)
+    const uint64_t col_tiles = (cols + TB - 1) / TB;
+    const uint32_t tb = VEC == 1 ? (uint32_t)((cols + col_tiles - 1) / col_tiles) : TB;
+    const uint64_t tiles_i = n / TI, n_tiles = tiles_i * ((cols + tb - 1) / tb);
     const uint64_t ctas = std::min<uint64_t>(n_tiles, (uint64_t)c.sm_count * per_sm);
-    transpose_rev_bulk_kernel<TI, TB, ST><<<(unsigned)ctas, G::THREADS, G::SMEM_BYTES, c.stream>>>(
-        in, out, lg, cols, tiles_i, n_tiles, c.wait_status(), extra, wait_ns);
+    transpose_rev_bulk_kernel<TI, TB, ST, VEC><<<(unsigned)ctas, G::THREADS, G::SMEM_BYTES, c.stream>>>(
+        in, out, lg, cols, tb, tiles_i, n_tiles, c.wait_status(), extra, wait_ns);
+}
+
+// Where the 8-byte bulk form is used: from 2^23 words on, whose input and output
+// no longer fit the 126 MB L2 (135 x 2^18: 140 against 200 us for the 8-byte
+// register form; 135 x 2^15, resident in L2: 28 against 23), and for up to 8
+// columns from 2^18 words on, which leave most of the register form's
+// 32-column tile empty (1 x 2^18: 23.7 against 26.5; 7 x 2^10: 13.5 against 13.3).
+static bool bulk8_pays(uint32_t lg, uint64_t cols)
+{
+    const uint64_t words = cols << lg;
+    return words >= (1ULL << 23) || (cols <= 8 && words >= (1ULL << 18));
 }
 
 void transpose_rev_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint32_t lg, uint64_t cols)
@@ -676,9 +692,13 @@ void transpose_rev_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint3
     // 9 (default) by column count: 64 x 64 tiles with 3 stages from 48
     // columns, else 64 x 32 with 4 (measured on B200: 0.198 against 0.213 ms
     // for the 16-byte form at 256 x 2^18, 0.223 against 0.240 ms at 16 x 2^22)
-    uint64_t form = vec16 ? tune_get("transpose_bulk", lg, 9) : 0;
+    // Odd column counts and destinations aligned to 8 bytes alone: the same
+    // tiles with 8-byte stores, unless the knob is 0.
+    const bool bulk8 = !vec16 && lg >= 6 && bulk8_pays(lg, cols) && ((uintptr_t)in % 16) == 0;
+    uint64_t form = vec16 || bulk8 ? tune_get("transpose_bulk", lg, 9) : 0;
     if (form == 9) form = cols >= 48 ? 3 : 1;
-    if (form >= 1 && form <= 8 && lg >= (form == 4 || form == 5 ? 7u : 6u)) {
+    const bool wide8 = bulk8 && form != 0;
+    if (wide8 || (form >= 1 && form <= 8 && lg >= (form == 4 || form == 5 ? 7u : 6u))) {
         uint32_t extra = 0;
         uint64_t wait_ns = 1000000000ULL;  // 1 s: a stage of tens of KiB lands in microseconds
         if (c.inject_wait_timeouts) {
@@ -686,7 +706,10 @@ void transpose_rev_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint3
             extra = 16;
             wait_ns = 20000000ULL;
         }
-        switch (form) {
+        const bool tall = form == 3 || form == 7 || form == 8;  // 64 columns a tile
+        if (wide8 && tall) launch_transpose_bulk<64, 64, 3, 1>(c, out, in, lg, cols, extra, wait_ns);
+        else if (wide8) launch_transpose_bulk<64, 32, 4, 1>(c, out, in, lg, cols, extra, wait_ns);
+        else switch (form) {
         case 1: launch_transpose_bulk<64, 32, 4>(c, out, in, lg, cols, extra, wait_ns); break;
         case 2: launch_transpose_bulk<64, 32, 2>(c, out, in, lg, cols, extra, wait_ns); break;
         case 3: launch_transpose_bulk<64, 64, 3>(c, out, in, lg, cols, extra, wait_ns); break;

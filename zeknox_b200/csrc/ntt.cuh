@@ -527,7 +527,12 @@ static __global__ void __launch_bounds__(256) transpose_rev_v2_kernel(const uint
 // mbarrier.  The threads then write the tile as bit-reversed leaf rows: a warp
 // writes 4 rows x 8 column pairs, 128 contiguous bytes per row, and reads the
 // stage without bank conflicts (words 8m + 2r mod 32 over pairs m < 4, rows
-// r < 4).  Needs n >= TI, an even column count and 16-byte aligned buffers.  A
+// r < 4).  With VEC = 1, for odd column counts and destinations aligned to 8
+// bytes, a thread stores one word: a warp writes 2 rows x 16 columns, each half
+// warp 8 columns x 2 rows so that its reads (words 2c + r mod 16) are free of
+// bank conflicts too.  The columns are dealt out evenly, tb <= TB per tile.
+// Needs n >= TI and a 16-byte aligned source (VEC = 2: also an even column
+// count, an even tb and a 16-byte aligned destination).  A
 // stage that is not complete after wait_ns sets *status and the CTA stops
 // (after waiting, bounded again, for the copies it has in flight); extra_tx > 0
 // declares that many bytes more than CTA 0's first tile delivers (a test of
@@ -540,16 +545,17 @@ struct TrBulk {
     static_assert(TB % 16 == 0 && TI % 4 == 0 && (TI * TB / 2) % THREADS == 0, "tile shape");
 };
 
-template <uint32_t TI, uint32_t TB, uint32_t STAGES>
+template <uint32_t TI, uint32_t TB, uint32_t STAGES, int VEC>
 static __global__ void __launch_bounds__(256)
     transpose_rev_bulk_kernel(const uint64_t *__restrict__ in, uint64_t *__restrict__ out, uint32_t lg, uint64_t cols,
-                              uint64_t tiles_i, uint64_t n_tiles, unsigned *status, uint32_t extra_tx, uint64_t wait_ns)
+                              uint32_t tb, uint64_t tiles_i, uint64_t n_tiles, unsigned *status, uint32_t extra_tx, uint64_t wait_ns)
 {
     using G = TrBulk<TI, TB, STAGES>;
     constexpr uint32_t THREADS = G::THREADS, PITCH = G::PITCH, STAGE_WORDS = G::STAGE_WORDS;
     extern __shared__ __align__(128) uint64_t stage_buf[];
     __shared__ __align__(8) uint64_t full[STAGES];
     const uint64_t n = 1ULL << lg;
+    const uint32_t blocks = (uint32_t)(n_tiles / tiles_i);  // of columns
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
 #pragma unroll
@@ -562,8 +568,8 @@ static __global__ void __launch_bounds__(256)
         const uint64_t t = blockIdx.x + k * gridDim.x;
         if (t >= n_tiles) return;
         const uint32_t s = (uint32_t)(k % STAGES);
-        const uint64_t i0 = (t % tiles_i) * TI, b0 = (t / tiles_i) * TB;
-        const uint32_t nb = (uint32_t)(cols - b0 < TB ? cols - b0 : TB);
+        const uint64_t i0 = (VEC == 1 ? t / blocks : t % tiles_i) * TI, b0 = (VEC == 1 ? t % blocks : t / tiles_i) * tb;
+        const uint32_t nb = (uint32_t)(cols - b0 < tb ? cols - b0 : tb);
         const uint32_t bar = smem_u32(&full[s]);
         if (lane == 0) mbar_arrive_expect_tx(bar, nb * TI * 8 + (k == 0 && blockIdx.x == 0 ? extra_tx : 0));
         __syncwarp();
@@ -587,16 +593,29 @@ static __global__ void __launch_bounds__(256)
             failed = true;
             break;
         }
-        const uint64_t i0 = (t % tiles_i) * TI, b0 = (t / tiles_i) * TB;
+        const uint64_t i0 = (VEC == 1 ? t / blocks : t % tiles_i) * TI, b0 = (VEC == 1 ? t % blocks : t / tiles_i) * tb;
         const uint64_t *tile = stage_buf + s * STAGE_WORDS;
+        const uint32_t nb = (uint32_t)(cols - b0 < tb ? cols - b0 : tb);
+        if constexpr (VEC == 1) {
+            // warps take whole runs of 2 rows: the row's columns, 16 at a time
+            const uint32_t c0 = (lane & 7) + ((lane >> 4) << 3), r0 = (lane >> 3) & 1;
+#pragma unroll 2
+            for (uint32_t r = 2 * warp + r0; r < TI; r += 2 * (THREADS / 32)) {
+                const uint64_t o = bitrev64(i0 + r, lg) * cols + b0;
+#pragma unroll
+                for (uint32_t c = c0; c < TB; c += 16)
+                    if (c < nb && ZK_IN_BOUNDS(o + c, n * cols, OOB_TRANSPOSE_OUT)) out[o + c] = tile[c * PITCH + r];
+            }
+        }
+        if constexpr (VEC == 2)
 #pragma unroll
         for (uint32_t q = 0; q < TI * TB / 2 / THREADS; q++) {
             const uint32_t u = tid + q * THREADS, w = u >> 5, l = u & 31;
             const uint32_t r = 4 * (w / (TB / 16)) + (l >> 3), c = 2 * (8 * (w % (TB / 16)) + (l & 7));
             const uint64_t b = b0 + c;
             const uint64_t oi = bitrev64(i0 + r, lg) * cols + b;
-            // b even and cols even: b + 1 < cols too
-            if (b < cols && ZK_IN_BOUNDS(oi + 1, n * cols, OOB_TRANSPOSE_OUT)) {
+            // c even and nb even: c + 1 < nb too
+            if (c < nb && ZK_IN_BOUNDS(oi + 1, n * cols, OOB_TRANSPOSE_OUT)) {
                 ulonglong2 v;
                 v.x = tile[c * PITCH + r];
                 v.y = tile[(c + 1) * PITCH + r];
