@@ -64,12 +64,12 @@ static bool direct_io(uint32_t logr, const NttPassArgs &a, bool rows)
 template <int INV, int LOADM, int STOREM>
 static void launch_pass(uint32_t logr, const NttPassArgs &a, uint64_t grid, uint32_t smem, cudaStream_t s)
 {
-    const bool direct = direct_io(logr, a, STOREM == STORE_ROWS);
+    const bool direct = STOREM != STORE_NATURAL && direct_io(logr, a, STOREM == STORE_ROWS);
     // row-output passes never exceed MAX_ROWS_LOGR (plan_passes): no kernels above it
 #define ZK_R(r) ((STOREM == STORE_ROWS && (r) > (int)MAX_ROWS_LOGR) ? (int)MAX_ROWS_LOGR : (r))
 #define ZK_CASE(r)                                                                       \
     case r:                                                                              \
-        if (direct) launch_one<ZK_R(r), INV, LOADM, STOREM, 1>(a, grid, smem, s);        \
+        if (direct) launch_one<ZK_R(r), INV, LOADM, STOREM, STOREM != STORE_NATURAL>(a, grid, smem, s); \
         else launch_one<ZK_R(r), INV, LOADM, STOREM, 0>(a, grid, smem, s);               \
         break;
     switch (logr) {
@@ -247,6 +247,44 @@ static void reorder(DeviceCtx &c, const uint64_t *src, uint64_t src_stride, uint
     ZK_CUDA(cudaGetLastError());
 }
 
+// Whether column transforms of 2^L points take one pass, whose CTAs then hold a
+// whole virtual column and write it in natural order themselves: no scratch and
+// no reorder launch.
+static bool one_pass(uint32_t L) { return plan_passes(L, false).size() == 1; }
+
+// A one-pass job with natural-order output, times mul and tab_out.
+static void run_natural(DeviceCtx &c, const DifJob &j, uint64_t mul, const uint64_t *tab_out)
+{
+    const uint64_t n = 1ULL << j.L;
+    NttPassArgs a{};
+    a.src = j.src;
+    a.src_stride = j.src_stride;
+    a.src_len = j.src_len;
+    a.tab = j.tab;
+    a.tab_len = j.tab_len;
+    a.n_src = j.n_src;
+    a.tw_small = c.twiddles(12, j.inverse);
+    a.vcols = j.vcols;
+    a.L = j.L;
+    a.rate = j.rate;
+    a.dst = j.dst;
+    a.dst_stride = j.dst_stride;
+    a.dst_len = j.dst_len;
+    a.mul = mul;
+    a.tab_out = tab_out;
+    if (j.vcols > 0x7FFFFFFFULL) throw arg_failure("transform batch too large for one launch");
+    const uint32_t smem = (uint32_t)n * 8;
+    if (j.inverse) {
+        if (j.load == LOAD_EXTEND) launch_pass<1, LOAD_EXTEND, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
+        else launch_pass<1, LOAD_PLAIN, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
+    } else {
+        if (j.load == LOAD_COSETS) launch_pass<0, LOAD_COSETS, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
+        else if (j.load == LOAD_SCALE) launch_pass<0, LOAD_SCALE, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
+        else launch_pass<0, LOAD_PLAIN, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
+    }
+    ZK_CUDA(cudaGetLastError());
+}
+
 // --------------------------------------------------------------- public ops
 
 void ntt_batch_device(DeviceCtx &c, uint64_t *inout, uint32_t lg, uint64_t batches, bool inverse, bool with_coset,
@@ -255,44 +293,33 @@ void ntt_batch_device(DeviceCtx &c, uint64_t *inout, uint32_t lg, uint64_t batch
     NvtxRange range("zeknox ntt");
     const uint64_t n = 1ULL << lg;
     if (batches == 0) return;
+    DifJob j{};
+    j.src = inout;
+    j.src_stride = n;
+    j.load = !inverse && with_coset ? LOAD_SCALE : LOAD_PLAIN;
+    const uint64_t *coset = with_coset ? c.coset_powers(lg) : nullptr;
+    j.tab = inverse ? nullptr : coset;
+    j.dst_stride = n;
+    j.vcols = batches;
+    j.L = lg;
+    j.inverse = inverse;
+    j.src_len = j.dst_len = n * batches;
+    j.tab_len = n;
+    // reference order: coset multiply (forward powers) then n^-1 (ntt.cu:137-143)
+    const uint64_t mul = inverse ? H_SIZE_INV[lg] : 1, *tab_out = inverse ? coset : nullptr;
+    if (one_pass(lg)) {
+        j.dst = inout;
+        run_natural(c, j, mul, tab_out);
+        return;
+    }
     DevBuf tmp;
-    if (scratch) {
-        tmp.p = nullptr;
-    } else {
+    if (!scratch) {
         tmp.ctx = &c;
-        tmp.p = c.alloc(n * batches * 8);
+        scratch = tmp.p = c.alloc(n * batches * 8);
     }
-    uint64_t *tp = scratch ? scratch : tmp.p;
-    if (!inverse) {
-        DifJob j{};
-        j.src = inout;
-        j.src_stride = n;
-        j.load = with_coset ? LOAD_SCALE : LOAD_PLAIN;
-        j.tab = with_coset ? c.coset_powers(lg) : nullptr;
-        j.dst = tp;
-        j.dst_stride = n;
-        j.vcols = batches;
-        j.L = lg;
-        j.src_len = j.dst_len = n * batches;
-        j.tab_len = n;
-        run_dif(c, j);
-        reorder(c, tp, n, inout, n, lg, 0, batches, 1, nullptr, n * batches, n * batches);
-    } else {
-        DifJob j{};
-        j.src = inout;
-        j.src_stride = n;
-        j.load = LOAD_PLAIN;
-        j.dst = tp;
-        j.dst_stride = n;
-        j.vcols = batches;
-        j.L = lg;
-        j.inverse = true;
-        j.src_len = j.dst_len = n * batches;
-        run_dif(c, j);
-        // reference order: coset multiply (forward powers) then n^-1 (ntt.cu:137-143)
-        reorder(c, tp, n, inout, n, lg, 0, batches, H_SIZE_INV[lg], with_coset ? c.coset_powers(lg) : nullptr,
-                n * batches, n * batches);
-    }
+    j.dst = scratch;
+    run_dif(c, j);
+    reorder(c, scratch, n, inout, n, lg, 0, batches, mul, tab_out, n * batches, n * batches);
 }
 
 void lde_batch_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint32_t lg_n, uint32_t rate, uint64_t batches,
@@ -303,43 +330,44 @@ void lde_batch_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint32_t 
     const uint32_t lgN = lg_n + rate;
     const uint64_t N = 1ULL << lgN;
     if (batches == 0) return;
-    DevBuf tmp(c, N * batches);
+    DifJob j{};
+    j.src = in;
+    j.src_stride = n;
+    j.src_len = n * batches;
+    j.dst_len = N * batches;
+    uint64_t mul = 1;
+    const uint64_t *tab_out = nullptr;
     if (!inverse) {
         // coset c of column b is virtual column b*2^rate + c of size n
         const uint64_t g = with_coset ? (c.coset_powers(0), c.coset_gen) : 1;
-        DifJob j{};
-        j.src = in;
-        j.src_stride = n;
         j.load = LOAD_COSETS;
         j.tab = c.lde_table(lg_n, rate, g);
-        j.dst = tmp.p;
-        j.dst_stride = n;
         j.vcols = batches << rate;
         j.L = lg_n;
         j.rate = rate;
-        j.src_len = n * batches;
-        j.tab_len = N;
-        j.dst_len = N * batches;
-        run_dif(c, j);
-        reorder(c, tmp.p, n, out, N, lg_n, rate, batches, 1, nullptr, N * batches, N * batches);
     } else {
         // zero-extended inverse transform of size N (ntt.cu:529-535)
-        DifJob j{};
-        j.src = in;
-        j.src_stride = n;
         j.load = LOAD_EXTEND;
         j.n_src = n;
-        j.dst = tmp.p;
-        j.dst_stride = N;
         j.vcols = batches;
         j.L = lgN;
         j.inverse = true;
-        j.src_len = n * batches;
-        j.dst_len = N * batches;
-        run_dif(c, j);
-        reorder(c, tmp.p, N, out, N, lgN, 0, batches, H_SIZE_INV[lgN], with_coset ? c.coset_powers(lgN) : nullptr,
-                N * batches, N * batches);
+        mul = H_SIZE_INV[lgN];
+        tab_out = with_coset ? c.coset_powers(lgN) : nullptr;
     }
+    j.tab_len = N;
+    // (a column is read and written by different CTAs: no overlap of input and output)
+    if (one_pass(j.L) && (in + n * batches <= out || out + N * batches <= in)) {
+        j.dst = out;
+        j.dst_stride = N;
+        run_natural(c, j, mul, tab_out);
+        return;
+    }
+    DevBuf tmp(c, N * batches);
+    j.dst = tmp.p;
+    j.dst_stride = 1ULL << j.L;
+    run_dif(c, j);
+    reorder(c, tmp.p, j.dst_stride, out, N, j.L, j.rate, batches, mul, tab_out, N * batches, N * batches);
 }
 
 // Columns per chunk of the fused LDE: the intermediate of a chunk (2^(lg_n +

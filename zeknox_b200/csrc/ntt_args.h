@@ -14,6 +14,8 @@ enum NttLoad : int {
 
 enum NttStore : int {
     STORE_SAME = 0,      // dst[v * dst_stride + position]
+    STORE_NATURAL = 2,   // dst[(v >> rate) * dst_stride + (i << rate) + (v & (2^rate-1))], i natural, times mul
+                         // and tab_out (one-pass transforms: a tile is a whole virtual column)
     STORE_ROWS = 1,      // leaf-major: dst[(rev_rate(v & mask) * n + position) * cols + (v >> rate)]
 };
 
@@ -38,6 +40,9 @@ struct NttPassArgs {
     uint64_t *const *dst_tab;
     uint32_t log_rows_per_dst;
     uint64_t col_offset;
+    // STORE_NATURAL: factor of every output (1: none) and of output i of a column (null: none)
+    uint64_t mul;
+    const uint64_t *tab_out;
     // extents in words of src, dst (each destination buffer for dst_tab) and
     // tab from the pass's first element on: read only by the checked build
     uint64_t src_len, dst_len, tab_len;
