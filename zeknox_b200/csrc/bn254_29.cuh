@@ -132,6 +132,37 @@ static __device__ __noinline__ Fr29 fr29_dot5(int c0, int step, const Fr29 s0, c
 
 __device__ __forceinline__ Fr29 fr29_exp5(const Fr29 &x) { return fr29_mul(fr29_sqr(fr29_sqr(x)), x); }
 
+// Out of Montgomery form, canonical, the low 192 bits as three lanes (most
+// significant word first), each reduced once mod p.
+__device__ __forceinline__ void fr29_words(const Fr29 &x, uint64_t s[3])
+{
+    Fr29 one;
+#pragma unroll
+    for (int k = 0; k < 9; k++) one.w[k] = k == 0;
+    const Fr29 v = fr29_mul(x, one);  // at most r
+    Fr29 d;                           // v - r when v >= r
+    uint32_t borrow = 0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const uint32_t t = v.w[k] - fr29_r(k) - borrow;
+        borrow = t >> 31;
+        d.w[k] = t & FR29_MASK;
+    }
+#pragma unroll
+    for (int k = 0; k < 9; k++) d.w[k] = borrow ? v.w[k] : d.w[k];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        uint64_t limb = 0;
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+            const int at = 29 * j - 64 * k;  // limb j's first bit in this word
+            if (at > -29 && at < 0) limb |= (uint64_t)d.w[j] >> -at;
+            else if (at >= 0 && at < 64) limb |= (uint64_t)d.w[j] << at;
+        }
+        s[2 - k] = gl_canon(limb);
+    }
+}
+
 // poseidon_bn128_permute (hash.cuh) on the 12 Goldilocks lanes.
 __device__ __forceinline__ void poseidon_bn128_permute29(uint64_t s[12])
 {
@@ -186,33 +217,121 @@ __device__ __forceinline__ void poseidon_bn128_permute29(uint64_t s[12])
         }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        Fr29 one;
+    for (int i = 0; i < 4; i++) fr29_words(st[i], s + 3 * i);
+}
+
+// ---- one state per five threads.  A permutation on one thread is about 1 M
+// cycles, which the narrow levels of a tree and forests of a few thousand
+// leaves wait on.  Here thread i < 5 of a group holds state slot i, six groups
+// to a warp (threads 30 and 31 repeat a group that does not exist): the S-boxes
+// of a full round run side by side, and of a partial round's products only the
+// three of slot 0's S-box and one more are in sequence.  All 32 threads call
+// together.
+struct Fr29Group {
+    uint32_t i, base;  // slot, first thread of the group
+    bool live;
+    __device__ __forceinline__ void init()
+    {
+        const uint32_t lane = threadIdx.x & 31u;
+        i = lane % 5;
+        base = lane - i;
+        live = lane < 30;
+    }
+};
+
+// constants read at another index by every thread: the constant bank would
+// serialise them
+static __device__ const uint32_t g_FR29[ZK_FR29_WORDS] = {ZK_FR29_LIST};
+
+__device__ __forceinline__ Fr29 fr29_const_g(int idx)
+{
+    Fr29 z;
 #pragma unroll
-        for (int k = 0; k < 9; k++) one.w[k] = k == 0;
-        const Fr29 v = fr29_mul(st[i], one);  // at most r
-        // v - r when v >= r
-        Fr29 d;
-        uint32_t borrow = 0;
+    for (int k = 0; k < 9; k++) z.w[k] = __ldg(&g_FR29[9 * idx + k]);
+    return z;
+}
+
+// slot j's element, in every thread of the group
+__device__ __forceinline__ Fr29 fr29_from(const Fr29 &a, const Fr29Group &g, uint32_t j)
+{
+    Fr29 z;
+#pragma unroll
+    for (int k = 0; k < 9; k++) z.w[k] = __shfl_sync(0xFFFFFFFFu, a.w[k], (g.base + j) & 31u);
+    return z;
+}
+
+// s: lanes 3 (i - 1) .. 3 (i - 1) + 2 of the state in threads 1..4.  Bounds as
+// above, but for slot 0 in the partial rounds: a sum of five reduced products,
+// below 7 r.
+__device__ __forceinline__ void poseidon_bn128_permute_group(uint64_t s[3], const Fr29Group &g)
+{
+    Fr29 st;
+    {
+        const uint64_t l[3] = {gl_canon(s[2]), gl_canon(s[1]), gl_canon(s[0])};
+        Fr29 x;
 #pragma unroll
         for (int k = 0; k < 9; k++) {
-            const uint32_t t = v.w[k] - fr29_r(k) - borrow;
-            borrow = t >> 31;
-            d.w[k] = t & FR29_MASK;
+            const int bit = 29 * k, q = bit >> 6, sh = bit & 63;
+            uint64_t v = q < 3 ? l[q] >> sh : 0;
+            if (sh > 35 && q + 1 < 3) v |= l[q + 1] << (64 - sh);
+            x.w[k] = g.i ? (uint32_t)v & FR29_MASK : 0;
         }
+        st = fr29_add(fr29_mul(x, fr29_const_g(FR29_R2)), fr29_const_g(FR29_C + g.i));
+    }
+#pragma unroll 1
+    for (int f = 0; f < 8; f++) {
+        st = fr29_exp5(st);
+        if (f != 7) st = fr29_add(st, fr29_const_g(FR29_C + (f < 4 ? 5 * (f + 1) : 85 + 5 * (f - 4)) + g.i));
+        uint64_t c[17] = {};
+        const int m0 = (f == 3 ? FR29_P : FR29_M) + g.i;
+#pragma unroll 1
+        for (int j = 0; j < 5; j++) fr29_columns_add(c, fr29_from(st, g, j), fr29_const_g(m0 + 5 * j));
+        st = fr29_montgomery(c);
+        if (f == 3) {
+#pragma unroll 1
+            for (int r = 0; r < 60; r++) {
+                const int row = FR29_S + 9 * r;
+                // slot 0 squares, the others take their term of its row
+                const Fr29 sk = fr29_const_g(row + g.i);
+                Fr29 b;
 #pragma unroll
-        for (int k = 0; k < 9; k++) d.w[k] = borrow ? v.w[k] : d.w[k];
+                for (int k = 0; k < 9; k++) b.w[k] = g.i ? sk.w[k] : st.w[k];
+                const Fr29 p = fr29_mul(st, b);
+                const Fr29 x5 = fr29_mul(fr29_sqr(p), st);
+                const Fr29 x0 = fr29_from(fr29_add(x5, fr29_const_g(FR29_C + 25 + r)), g, 0);
+                const Fr29 v = fr29_mul(x0, fr29_const_g(g.i ? row + 4 + g.i : row));
+                const Fr29 next = fr29_add(st, v);  // slots 1..4
+                Fr29 sum = v;                       // slot 0
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            uint64_t limb = 0;
+                for (uint32_t j = 1; j < 5; j++) {
+                    const Fr29 t = fr29_from(p, g, j);
 #pragma unroll
-            for (int j = 0; j < 9; j++) {
-                const int at = 29 * j - 64 * k;  // limb j's first bit in this word
-                if (at > -29 && at < 0) limb |= (uint64_t)d.w[j] >> -at;
-                else if (at >= 0 && at < 64) limb |= (uint64_t)d.w[j] << at;
+                    for (int k = 0; k < 9; k++) sum.w[k] += t.w[k];
+                }
+                fr29_carry(sum);
+#pragma unroll
+                for (int k = 0; k < 9; k++) st.w[k] = g.i ? next.w[k] : sum.w[k];
             }
-            s[3 * i + 2 - k] = gl_canon(limb);
         }
+    }
+    // slots 0..3 go to the elements of threads 1..4
+    st = fr29_from(st, g, (g.i + 4) % 5);
+    fr29_words(st, s);
+}
+
+// Plonky2's sponge (hash.cuh sponge_hash_one) with the state in the group; all
+// threads of a group pass the same src and len > 4.  Digest words 0..2 are left
+// in thread 1's out, word 3 in thread 2's out[0].
+__device__ __forceinline__ void sponge_bn128_group(const uint64_t *src, uint64_t len, uint64_t out[3], const Fr29Group &g)
+{
+    out[0] = out[1] = out[2] = 0;
+    const uint32_t l0 = g.i ? 3 * (g.i - 1) : 12;  // this thread's first lane
+#pragma unroll 1
+    for (uint64_t idx = 0; idx < len; idx += 8) {
+#pragma unroll
+        for (uint32_t q = 0; q < 3; q++)
+            if (l0 + q < 8 && idx + l0 + q < len) out[q] = src[idx + l0 + q];
+        poseidon_bn128_permute_group(out, g);
     }
 }
 

@@ -6,9 +6,10 @@
 // has >= wide_level_nodes nodes; then folds inside CTAs.  Poseidon, Poseidon2
 // and Monolith run their linear layers on the tensor cores (hash_mma.cuh), 32,
 // 16 or 8 leaves per warp by the forest's size, and fold 6 levels per launch
-// until a CTA holds whole subtrees.  Keccak and Poseidon-BN128 hash one leaf
-// or node per thread: a fold kernel of 8 levels and, for subtrees still above
-// 1024 nodes, level kernels, then one tail CTA per subtree.
+// until a CTA holds whole subtrees; so does Poseidon-BN128, five threads a
+// state in small forests and narrow levels.  Keccak hashes one leaf or node per
+// thread: a fold kernel of 8 levels and, for subtrees still above 1024 nodes,
+// level kernels, then one tail CTA per subtree.
 #define ZK_BN128_LIMBS29 1
 #include <algorithm>
 #include <cstdio>
@@ -64,6 +65,11 @@ constexpr uint64_t mid_leaves()
 static constexpr uint64_t WIDE_LEVEL_NODES = 1ULL << 15;  // default: levels at least this wide run node-parallel
                                                           // ("wide_level_nodes.<hash>")
 
+// Poseidon-BN128 forests up to this many leaves hash them with five threads a
+// state ("coop_leaves.2"): 2^12 x 135 7.2 against 11.0 ms with one, 2^13 9.6
+// against 11.2, 2^14 13.7 against 11.3.
+static constexpr uint64_t BN128_COOP_LEAVES = 1ULL << 13;
+
 bool merkle_geometry_ok(uint64_t n_digests, uint64_t n_caps, uint64_t n_leaves, uint64_t cap_height, std::string &err)
 {
     return merkle_geometry_check(n_digests, n_caps, n_leaves, cap_height, err);
@@ -117,6 +123,9 @@ static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *lea
             else if (g.n_leaves <= mid_leaves<H>() * coop) launch_leaf_mma<H, 2>(lt, digests, caps, leaves, g, s);
             else launch_leaf_mma<H, 4>(lt, digests, caps, leaves, g, s);
         }
+    } else if (H == HASH_POSEIDON_BN128 && g.leaf_size > 4 &&
+               g.n_leaves <= tune_get("coop_leaves.2", lg_leaves, BN128_COOP_LEAVES)) {
+        merkle_leaf_bn128_kernel<64><<<(unsigned)((g.n_leaves + 11) / 12), 64, 0, s>>>(leaves, digests, caps, g);
     } else if (lt == 64) {
         blocks = (g.n_leaves + 63) / 64;
         merkle_leaf_kernel<H, 64><<<(unsigned)blocks, 64, 0, s>>>(leaves, digests, caps, g);
@@ -139,10 +148,12 @@ static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *lea
     }
     // Narrow levels: folded inside CTAs of fold_nodes nodes; the tensor-core
     // form repeats until its CTAs hold whole subtrees.
-    if constexpr (HasMma<H>::value) {
+    if constexpr (HasMma<H>::value || H == HASH_POSEIDON_BN128) {
         for (;;) {
             const uint64_t count = g.n_leaves >> u0;
-            merkle_fold_mma_kernel<H><<<(unsigned)((count + MMA_FOLD_IN - 1) / MMA_FOLD_IN), 128, 0, s>>>(digests, caps, g, u0);
+            const unsigned ctas = (unsigned)((count + MMA_FOLD_IN - 1) / MMA_FOLD_IN);
+            if constexpr (HasMma<H>::value) merkle_fold_mma_kernel<H><<<ctas, 128, 0, s>>>(digests, caps, g, u0);
+            else merkle_fold_bn128_kernel<<<ctas, 192, 0, s>>>(digests, caps, g, u0);
             note_launch();
             if ((g.sub_leaves >> u0) <= MMA_FOLD_IN) return;  // caps written
             u0 += __builtin_ctz(MMA_FOLD_IN);

@@ -339,4 +339,96 @@ __global__ void __launch_bounds__(128) merkle_fold_mma_kernel(uint64_t *__restri
     }
 }
 
+#if ZK_BN128_LIMBS29
+// ---------------------------------------------- Poseidon-BN128, five threads a state
+//
+// (bn254_29.cuh.)  Groups without a leaf or node repeat their warp's last one
+// and store nothing.
+
+// Leaf digests (leaf_size > 4), six per warp.
+template <int T>
+__global__ void __launch_bounds__(T)
+    merkle_leaf_bn128_kernel(const uint64_t *__restrict__ leaves, uint64_t *__restrict__ digests,
+                             uint64_t *__restrict__ caps, MerkleGeom g)
+{
+    Fr29Group grp;
+    grp.init();
+    const uint64_t first = ((uint64_t)blockIdx.x * (T / 32) + (threadIdx.x >> 5)) * 6;
+    if (first >= g.n_leaves) return;  // the whole warp is past the end
+    const uint64_t i = first + grp.base / 5;
+    const bool act = grp.live && i < g.n_leaves;
+    const uint64_t row = act ? i : first;
+    const bool ok = ZK_IN_BOUNDS((row + 1) * g.leaf_size - 1, merkle_leaf_words(g), OOB_MERKLE_LEAF);
+    uint64_t d[3];
+    sponge_bn128_group(leaves + (ok ? row : 0) * g.leaf_size, g.leaf_size, d, grp);
+    if (!act || !ok || grp.i == 0 || grp.i > 2) return;
+#pragma unroll
+    for (uint32_t q = 0; q < 3; q++) {
+        const uint64_t w = 3 * (grp.i - 1) + q;  // digest word
+        if (w > 3) continue;
+        if (g.sub_leaves == 1) {
+            if (ZK_IN_BOUNDS(4 * i + w, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)) caps[4 * i + w] = d[q];
+        } else {
+            const uint64_t at = 4 * merkle_node_index(g, i, 0) + w;
+            if (ZK_IN_BOUNDS(at, merkle_digest_words(g), OOB_MERKLE_DIGEST)) digests[at] = d[q];
+        }
+    }
+}
+
+// merkle_fold_mma_kernel with five threads a state: six warps, 36 groups for
+// the 32 nodes of a CTA's first level.
+static __global__ void __launch_bounds__(192)
+    merkle_fold_bn128_kernel(uint64_t *__restrict__ digests, uint64_t *__restrict__ caps, MerkleGeom g, uint32_t u0)
+{
+    __shared__ uint64_t node[MMA_FOLD_IN][4];
+    Fr29Group grp;
+    grp.init();
+    const uint32_t wf = (threadIdx.x >> 5) * 6, quint = wf + grp.base / 5;  // first group of the warp, this group
+    const uint64_t count = g.n_leaves >> u0;
+    const uint64_t i0 = (uint64_t)blockIdx.x * MMA_FOLD_IN;
+    const uint64_t cta_nodes = count - i0 < MMA_FOLD_IN ? count - i0 : MMA_FOLD_IN;
+    for (uint32_t k = threadIdx.x; k < 4 * cta_nodes; k += 192) {
+        const uint64_t wi = 4 * merkle_node_index(g, (i0 + (k >> 2)) << u0, u0) + (k & 3);
+        node[k >> 2][k & 3] = ZK_IN_BOUNDS(wi, merkle_digest_words(g), OOB_MERKLE_NODE) ? digests[wi] : 0;
+    }
+    const uint32_t top = g.log_sub - 1;
+    uint32_t U = 0;
+    while ((1u << (U + 1)) <= MMA_FOLD_IN && u0 + U + 1 <= top) U++;
+    const uint64_t sub_nodes = g.sub_leaves >> u0;
+    const uint32_t last = u0 + U == top && sub_nodes <= MMA_FOLD_IN ? U + 1 : U;
+#pragma unroll 1
+    for (uint32_t v = 1; v <= last; v++) {
+        __syncthreads();
+        const uint32_t nodes = v <= U ? (uint32_t)((cta_nodes + (1u << v) - 1) >> v) : (uint32_t)(cta_nodes / sub_nodes);
+        const bool act = grp.live && quint < nodes;
+        uint64_t h[3];
+        if (wf < nodes) {
+            sponge_bn128_group(&node[2 * (act ? quint : wf)][0], 8, h, grp);
+            if (act && (grp.i == 1 || grp.i == 2)) {
+#pragma unroll
+                for (uint32_t q = 0; q < 3; q++) {
+                    const uint32_t w = 3 * (grp.i - 1) + q;
+                    if (w > 3) continue;
+                    if (v <= U) {
+                        const uint64_t at = 4 * merkle_node_index(g, (i0 + ((uint64_t)quint << v)) << u0, u0 + v) + w;
+                        if (ZK_IN_BOUNDS(at, merkle_digest_words(g), OOB_MERKLE_DIGEST)) digests[at] = h[q];
+                    } else {
+                        const uint64_t at = 4 * (((i0 << u0) >> g.log_sub) + quint) + w;
+                        if (ZK_IN_BOUNDS(at, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)) caps[at] = h[q];
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (act && v <= U && (grp.i == 1 || grp.i == 2)) {
+#pragma unroll
+            for (uint32_t q = 0; q < 3; q++) {
+                const uint32_t w = 3 * (grp.i - 1) + q;
+                if (w <= 3) node[quint][w] = h[q];
+            }
+        }
+    }
+}
+#endif  // ZK_BN128_LIMBS29
+
 }  // namespace zk
