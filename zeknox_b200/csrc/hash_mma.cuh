@@ -42,6 +42,9 @@ static __device__ const __align__(16) uint32_t g_mma_monolith[MMA_MONO_WORDS] = 
 static __device__ const uint64_t g_mma_rc0[12] = {ZK_MMA_POSEIDON_RC0};  // Poseidon's first constants
 
 template <int H>
+constexpr uint32_t mma_table_words() { return H == HASH_MONOLITH ? MMA_MONO_WORDS : MMA_WORDS; }
+
+template <int H>
 __device__ __forceinline__ const uint32_t *mma_table()
 {
     if constexpr (H == HASH_POSEIDON) return g_mma_poseidon;
@@ -146,8 +149,16 @@ __device__ __forceinline__ void mma_store_group(uint32_t *p, const uint64_t *v)
     for (int k = 0; k < M::TILES; k++) MmaA<NS>::store(p + k * M::TILE, v + M::ROWS * k);
 }
 
+// Table words through L1, or from a copy in shared memory (TSM).
+template <bool TSM>
+__device__ __forceinline__ uint4 mma_ld(const uint32_t *p)
+{
+    if constexpr (TSM) return *(const uint4 *)p;
+    else return __ldg((const uint4 *)p);
+}
+
 // Sums of one group of four output lanes.
-template <int NS>
+template <int NS, bool TSM>
 struct MmaAcc {
     using M = MmaSmem<NS>;
     uint32_t s[M::TILES][4][4];
@@ -155,7 +166,7 @@ struct MmaAcc {
     {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint4 v = __ldg((const uint4 *)(c + 16 * i));
+            const uint4 v = mma_ld<TSM>(c + 16 * i);
 #pragma unroll
             for (int k = 0; k < M::TILES; k++) {
                 s[k][i][0] = v.x;
@@ -167,7 +178,7 @@ struct MmaAcc {
     }
     __device__ __forceinline__ void add(const MmaA<NS> *a, const uint32_t *b)
     {
-        const uint4 p = __ldg((const uint4 *)b), q = __ldg((const uint4 *)(b + 128));
+        const uint4 p = mma_ld<TSM>(b), q = mma_ld<TSM>(b + 128);
 #pragma unroll
         for (int k = 0; k < M::TILES; k++) {
             const uint32_t *w = a[k].w;
@@ -180,7 +191,7 @@ struct MmaAcc {
     // += a full-round layer (mma_full_operands)
     __device__ __forceinline__ void add_full(const uint32_t (*a)[4][4], const uint32_t *b)
     {
-        const uint4 p = __ldg((const uint4 *)b), q = __ldg((const uint4 *)(b + 128));
+        const uint4 p = mma_ld<TSM>(b), q = mma_ld<TSM>(b + 128);
 #pragma unroll
         for (int k = 0; k < M::TILES; k++) {
             mma_16832(s[k][0], a[k][0][0], a[k][0][1], a[k][0][2], a[k][0][3], p.x, p.y, s[k][0]);
@@ -278,14 +289,14 @@ __device__ __forceinline__ void mma_full_operands(uint32_t (*x)[4][4], const uin
 
 // Block i < 6 of the partial rounds (four rounds, two in the last): 3 + i
 // k-blocks of operands, the S-box outputs into k-block 3 + i.
-template <int H, int NS>
+template <int H, int NS, bool TSM>
 __device__ __forceinline__ void mma_rounds4(uint32_t *sm, const uint32_t *b, const uint32_t *c, int i)
 {
     using M = MmaSmem<NS>;
     const uint32_t lane = threadIdx.x & 31, t = lane & 3, g = lane >> 2;
     const uint32_t q = t % NS;  // the state whose S-box chain this thread runs
     const uint32_t *a = sm + lane * 2 * M::ROWS;
-    MmaAcc<NS> acc;
+    MmaAcc<NS, TSM> acc;
     acc.start(c);
 #pragma unroll
     for (int kb = 0; kb < 3; kb++) acc.add_smem(a + kb * M::BLOCK, b + kb * MMA_KB);
@@ -334,21 +345,21 @@ __device__ __forceinline__ void mma_rounds4(uint32_t *sm, const uint32_t *b, con
 // permutation is ~1300 instructions: unrolled forms of ~3000 stalled on
 // instruction fetch.  A layer reads its operands into registers before its
 // first store, and a thread's slots are its own, so it works in place.
-template <int H, int NS>
-__device__ __forceinline__ void permute_mma(uint32_t *sm, uint32_t groups)
+template <int H, int NS, bool TSM = false>
+__device__ __forceinline__ void permute_mma(uint32_t *sm, uint32_t groups, const uint32_t *table = mma_table<H>())
 {
     using M = MmaSmem<NS>;
     const uint32_t lane = threadIdx.x & 31, t = lane & 3;
     constexpr int J = MmaSmem<NS>::GROUPS;
     uint32_t *a = sm + lane * 2 * M::ROWS;
-    const uint32_t *tab = mma_table<H>() + 4 * lane, *cst = mma_table<H>() + 4 * t;
+    const uint32_t *tab = table + 4 * lane, *cst = table + 4 * t;
 #pragma unroll 1
     for (int st = 0; st < 10; st++) {
         if (st == 4) {  // the partial rounds
             const uint32_t *b = tab + MMA_Y, *c = cst + MMA_YCONST;
 #pragma unroll 1
             for (int i = 0; i < 6; i++, c += MMA_GROUP) {
-                mma_rounds4<H, NS>(sm, b, c, i);
+                mma_rounds4<H, NS, TSM>(sm, b, c, i);
                 b += (3 + i) * MMA_KB;
             }
             b = tab + MMA_W;
@@ -360,7 +371,7 @@ __device__ __forceinline__ void permute_mma(uint32_t *sm, uint32_t groups)
                 for (int k = 0; k < M::TILES; k++) x[kb][k].load(a + kb * M::BLOCK + k * M::TILE);
 #pragma unroll 1
             for (int j0 = 0; j0 < 3; j0 += J, b += 9 * J * MMA_KB, c += J * MMA_GROUP) {
-                MmaAcc<NS> acc[J];
+                MmaAcc<NS, TSM> acc[J];
 #pragma unroll
                 for (int j = 0; j < J; j++) {
                     acc[j].start(c + j * MMA_GROUP);
@@ -402,7 +413,7 @@ __device__ __forceinline__ void permute_mma(uint32_t *sm, uint32_t groups)
                     }
                 }
             } else {
-                MmaAcc<NS> acc[J];
+                MmaAcc<NS, TSM> acc[J];
 #pragma unroll
                 for (int j = 0; j < J; j++) {
                     acc[j].start(c + j * MMA_GROUP);
@@ -450,8 +461,8 @@ __device__ __forceinline__ uint64_t mma_add_nc(uint64_t a, uint64_t b)
 // one the Bars act on, one lane per thread; Bricks take the square of lane
 // i - 1 from the thread before in the quad, or, for t = 0, the square of the
 // group before from thread 3.
-template <int NS>
-__device__ __forceinline__ void permute_mma_monolith(uint32_t *sm, uint32_t groups)
+template <int NS, bool TSM = false>
+__device__ __forceinline__ void permute_mma_monolith(uint32_t *sm, uint32_t groups, const uint32_t *table = g_mma_monolith)
 {
     using M = MmaSmem<NS>;
     constexpr int J = M::GROUPS;
@@ -461,8 +472,8 @@ __device__ __forceinline__ void permute_mma_monolith(uint32_t *sm, uint32_t grou
 #pragma unroll 1
     for (int st = 0; st < 7; st++) {
         const uint32_t mask = st == 6 ? groups : 7u;
-        const uint32_t *b = g_mma_monolith + MMA_FULL + 4 * lane;
-        const uint32_t *c = g_mma_monolith + MMA_MONO_CONST + 3 * MMA_GROUP * st + 4 * t;
+        const uint32_t *b = table + MMA_FULL + 4 * lane;
+        const uint32_t *c = table + MMA_MONO_CONST + 3 * MMA_GROUP * st + 4 * t;
         uint32_t x[M::TILES][4][4];
         mma_full_operands<NS>(x, a);
         uint64_t prev[NS];  // squares of the group before
@@ -471,7 +482,7 @@ __device__ __forceinline__ void permute_mma_monolith(uint32_t *sm, uint32_t grou
 #pragma unroll 1
         for (int j0 = 0; j0 < 3; j0 += J, b += J * MMA_KB, c += J * MMA_GROUP) {
             if (J == 1 && !((mask >> j0) & 1u)) continue;
-            MmaAcc<NS> acc[J];
+            MmaAcc<NS, TSM> acc[J];
             uint64_t v[J][NS];
 #pragma unroll
             for (int j = 0; j < J; j++) {
@@ -523,8 +534,9 @@ __device__ __forceinline__ void mma_set_lane(uint32_t *sm, int kb, int q, uint64
 
 // sponge_hash_one for the warp's states: row(q) is where state q's len words
 // are; the digest word t of state q is left in d[q] (canonical).  len > 4.
-template <int H, int NS, class Row>
-__device__ __forceinline__ void sponge_hash_mma(Row row, uint64_t len, uint32_t *sm, uint64_t d[NS])
+template <int H, int NS, bool TSM = false, class Row>
+__device__ __forceinline__ void sponge_hash_mma(Row row, uint64_t len, uint32_t *sm, uint64_t d[NS],
+                                                const uint32_t *table = mma_table<H>())
 {
     const uint32_t t = threadIdx.x & 3;
 #pragma unroll
@@ -543,8 +555,8 @@ __device__ __forceinline__ void sponge_hash_mma(Row row, uint64_t len, uint32_t 
         // k < 8 words also lanes k..7
         const uint64_t rem = len - idx;
         const uint32_t groups = rem <= 8 ? 1u : rem >= 16 ? 4u : rem >= 12 ? 6u : 7u;
-        if constexpr (H == HASH_MONOLITH) permute_mma_monolith<NS>(sm, groups);
-        else permute_mma<H, NS>(sm, groups);
+        if constexpr (H == HASH_MONOLITH) permute_mma_monolith<NS, TSM>(sm, groups, table);
+        else permute_mma<H, NS, TSM>(sm, groups, table);
     }
 #pragma unroll
     for (int q = 0; q < NS; q++) d[q] = gl_canon(mma_lane<NS>(sm, 0, q));

@@ -291,15 +291,25 @@ __global__ void __launch_bounds__(T, NS == 4 ? MMA_THREADS_PER_SM / T : 1)
 // permutation per quad of threads) and computes every node above them whose
 // subtree lies in the CTA, and the caps of subtrees that fit.  What these
 // narrow levels wait on is the latency of one permutation per level: 8 states
-// per warp (NS = 1), a third of the lanes' S-boxes per thread.
+// per warp (NS = 1), a third of the lanes' S-boxes per thread.  TSM: the tables
+// are copied to dynamic shared memory first, when a CTA has an SM to itself.
+// L1 starts empty at every launch, and a warp alone fetches the tables' lines
+// one after another on its first permutation.
 static constexpr uint32_t MMA_FOLD_IN = 64;
 
-template <int H>
+template <int H, bool TSM>
 __global__ void __launch_bounds__(128) merkle_fold_mma_kernel(uint64_t *__restrict__ digests, uint64_t *__restrict__ caps,
                                                               MerkleGeom g, uint32_t u0)
 {
+    extern __shared__ __align__(16) uint32_t table_copy[];
     __shared__ __align__(16) uint32_t sm[4][MmaSmem<1>::words<H>()];
     __shared__ uint64_t node[MMA_FOLD_IN][4];
+    if constexpr (TSM) {
+        const uint4 *table = (const uint4 *)mma_table<H>();
+#pragma unroll 12
+        for (uint32_t k = threadIdx.x; k < mma_table_words<H>() / 4; k += 128)
+            ((uint4 *)table_copy)[k] = __ldg(table + k);
+    }
     const uint32_t quad = threadIdx.x >> 2, t = threadIdx.x & 3, warp = threadIdx.x >> 5;
     const uint32_t wq = quad & ~7u;  // first quad of this warp
     const uint64_t count = g.n_leaves >> u0;
@@ -325,7 +335,8 @@ __global__ void __launch_bounds__(128) merkle_fold_mma_kernel(uint64_t *__restri
         if (wq < nodes) {
             // a quad with no node repeats its warp's first
             const uint64_t *src = &node[2 * (act ? quad : wq)][0];
-            sponge_hash_mma<H, 1>([&](int) { return src; }, 8, sm[warp], h);
+            if constexpr (TSM) sponge_hash_mma<H, 1, true>([&](int) { return src; }, 8, sm[warp], h, table_copy);
+            else sponge_hash_mma<H, 1>([&](int) { return src; }, 8, sm[warp], h);
             if (act && v <= U) {
                 const uint64_t w = 4 * merkle_node_index(g, (i0 + ((uint64_t)quad << v)) << u0, u0 + v) + t;
                 if (ZK_IN_BOUNDS(w, merkle_digest_words(g), OOB_MERKLE_DIGEST)) digests[w] = h[0];
