@@ -155,6 +155,12 @@ struct DifJob {
     // extents in words of src, dst (each scatter destination), tab and
     // scratch, read only by the checked build's range checks
     uint64_t src_len, dst_len, tab_len, scratch_len;
+    // natural-order output by the last pass (null: bit-reversed, at dst): at
+    // out, column stride out_stride, times mul (1: none) and tab_out (null:
+    // none); dst then holds the passes before it
+    uint64_t *out;
+    uint64_t out_stride, out_len, mul;
+    const uint64_t *tab_out;
 };
 
 static void run_dif(DeviceCtx &c, const DifJob &j)
@@ -194,6 +200,12 @@ static void run_dif(DeviceCtx &c, const DifJob &j)
                 a.log_rows_per_dst = j.scatter->log_rows_per_dst;
                 a.col_offset = j.scatter->col_offset + j.col0;
             }
+        } else if (j.out && last) {
+            a.dst = j.out;
+            a.dst_stride = j.out_stride;
+            a.dst_len = j.out_len;
+            a.mul = j.mul;
+            a.tab_out = j.tab_out;
         } else {
             a.dst = j.rows ? j.scratch : j.dst;
             a.dst_stride = j.rows ? n : j.dst_stride;
@@ -215,7 +227,16 @@ static void run_dif(DeviceCtx &c, const DifJob &j)
         if (grid == 0) continue;
         if (grid > 0x7FFFFFFFULL) throw arg_failure("transform batch too large for one launch");
         const uint32_t smem = tile * 8;
-        if (!j.inverse) {
+        if (j.out && last) {
+            if (j.inverse) {
+                if (load == LOAD_EXTEND) launch_pass<1, LOAD_EXTEND, STORE_NATURAL>(ps.logr, a, grid, smem, c.stream);
+                else launch_pass<1, LOAD_PLAIN, STORE_NATURAL>(ps.logr, a, grid, smem, c.stream);
+            } else {
+                if (load == LOAD_COSETS) launch_pass<0, LOAD_COSETS, STORE_NATURAL>(ps.logr, a, grid, smem, c.stream);
+                else if (load == LOAD_SCALE) launch_pass<0, LOAD_SCALE, STORE_NATURAL>(ps.logr, a, grid, smem, c.stream);
+                else launch_pass<0, LOAD_PLAIN, STORE_NATURAL>(ps.logr, a, grid, smem, c.stream);
+            }
+        } else if (!j.inverse) {
             if (store_rows) {
                 if (load == LOAD_COSETS) launch_pass<0, LOAD_COSETS, STORE_ROWS>(ps.logr, a, grid, smem, c.stream);
                 else launch_pass<0, LOAD_PLAIN, STORE_ROWS>(ps.logr, a, grid, smem, c.stream);
@@ -247,43 +268,8 @@ static void reorder(DeviceCtx &c, const uint64_t *src, uint64_t src_stride, uint
     ZK_CUDA(cudaGetLastError());
 }
 
-// Whether column transforms of 2^L points take one pass, whose CTAs then hold a
-// whole virtual column and write it in natural order themselves: no scratch and
-// no reorder launch.
+// Whether column transforms of 2^L points take one pass.
 static bool one_pass(uint32_t L) { return plan_passes(L, false).size() == 1; }
-
-// A one-pass job with natural-order output, times mul and tab_out.
-static void run_natural(DeviceCtx &c, const DifJob &j, uint64_t mul, const uint64_t *tab_out)
-{
-    const uint64_t n = 1ULL << j.L;
-    NttPassArgs a{};
-    a.src = j.src;
-    a.src_stride = j.src_stride;
-    a.src_len = j.src_len;
-    a.tab = j.tab;
-    a.tab_len = j.tab_len;
-    a.n_src = j.n_src;
-    a.tw_small = c.twiddles(12, j.inverse);
-    a.vcols = j.vcols;
-    a.L = j.L;
-    a.rate = j.rate;
-    a.dst = j.dst;
-    a.dst_stride = j.dst_stride;
-    a.dst_len = j.dst_len;
-    a.mul = mul;
-    a.tab_out = tab_out;
-    if (j.vcols > 0x7FFFFFFFULL) throw arg_failure("transform batch too large for one launch");
-    const uint32_t smem = (uint32_t)n * 8;
-    if (j.inverse) {
-        if (j.load == LOAD_EXTEND) launch_pass<1, LOAD_EXTEND, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
-        else launch_pass<1, LOAD_PLAIN, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
-    } else {
-        if (j.load == LOAD_COSETS) launch_pass<0, LOAD_COSETS, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
-        else if (j.load == LOAD_SCALE) launch_pass<0, LOAD_SCALE, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
-        else launch_pass<0, LOAD_PLAIN, STORE_NATURAL>(j.L, a, j.vcols, smem, c.stream);
-    }
-    ZK_CUDA(cudaGetLastError());
-}
 
 // --------------------------------------------------------------- public ops
 
@@ -299,27 +285,23 @@ void ntt_batch_device(DeviceCtx &c, uint64_t *inout, uint32_t lg, uint64_t batch
     j.load = !inverse && with_coset ? LOAD_SCALE : LOAD_PLAIN;
     const uint64_t *coset = with_coset ? c.coset_powers(lg) : nullptr;
     j.tab = inverse ? nullptr : coset;
-    j.dst_stride = n;
     j.vcols = batches;
     j.L = lg;
     j.inverse = inverse;
-    j.src_len = j.dst_len = n * batches;
+    j.src_len = j.dst_len = j.out_len = n * batches;
     j.tab_len = n;
+    j.out = inout;
+    j.dst_stride = j.out_stride = n;
     // reference order: coset multiply (forward powers) then n^-1 (ntt.cu:137-143)
-    const uint64_t mul = inverse ? H_SIZE_INV[lg] : 1, *tab_out = inverse ? coset : nullptr;
-    if (one_pass(lg)) {
-        j.dst = inout;
-        run_natural(c, j, mul, tab_out);
-        return;
-    }
+    j.mul = inverse ? H_SIZE_INV[lg] : 1;
+    j.tab_out = inverse ? coset : nullptr;
     DevBuf tmp;
-    if (!scratch) {
+    if (!scratch && !one_pass(lg)) {
         tmp.ctx = &c;
         scratch = tmp.p = c.alloc(n * batches * 8);
     }
     j.dst = scratch;
     run_dif(c, j);
-    reorder(c, scratch, n, inout, n, lg, 0, batches, mul, tab_out, n * batches, n * batches);
 }
 
 void lde_batch_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint32_t lg_n, uint32_t rate, uint64_t batches,
@@ -334,9 +316,7 @@ void lde_batch_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint32_t 
     j.src = in;
     j.src_stride = n;
     j.src_len = n * batches;
-    j.dst_len = N * batches;
-    uint64_t mul = 1;
-    const uint64_t *tab_out = nullptr;
+    j.mul = 1;
     if (!inverse) {
         // coset c of column b is virtual column b*2^rate + c of size n
         const uint64_t g = with_coset ? (c.coset_powers(0), c.coset_gen) : 1;
@@ -352,22 +332,28 @@ void lde_batch_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint32_t 
         j.vcols = batches;
         j.L = lgN;
         j.inverse = true;
-        mul = H_SIZE_INV[lgN];
-        tab_out = with_coset ? c.coset_powers(lgN) : nullptr;
+        j.mul = H_SIZE_INV[lgN];
+        j.tab_out = with_coset ? c.coset_powers(lgN) : nullptr;
     }
     j.tab_len = N;
-    // (a column is read and written by different CTAs: no overlap of input and output)
-    if (one_pass(j.L) && (in + n * batches <= out || out + N * batches <= in)) {
-        j.dst = out;
-        j.dst_stride = N;
-        run_natural(c, j, mul, tab_out);
-        return;
-    }
-    DevBuf tmp(c, N * batches);
-    j.dst = tmp.p;
+    j.dst_len = j.out_len = N * batches;
     j.dst_stride = 1ULL << j.L;
+    j.out = out;
+    j.out_stride = N;
+    DevBuf tmp;
+    if (!one_pass(j.L)) {
+        tmp.ctx = &c;
+        j.dst = tmp.p = c.alloc(N * batches * 8);
+    } else if (in < out + N * batches && out < in + n * batches) {
+        // one pass over overlapping buffers would read columns another CTA has
+        // written: bit-reversed to a temporary, then reordered
+        tmp.ctx = &c;
+        j.dst = tmp.p = c.alloc(N * batches * 8);
+        j.out = nullptr;
+    }
     run_dif(c, j);
-    reorder(c, tmp.p, j.dst_stride, out, N, j.L, j.rate, batches, mul, tab_out, N * batches, N * batches);
+    if (!j.out)
+        reorder(c, tmp.p, j.dst_stride, out, N, j.L, j.rate, batches, j.mul, j.tab_out, N * batches, N * batches);
 }
 
 // Columns per chunk of the fused LDE: the intermediate of a chunk (2^(lg_n +

@@ -14,8 +14,8 @@ enum NttLoad : int {
 
 enum NttStore : int {
     STORE_SAME = 0,      // dst[v * dst_stride + position]
-    STORE_NATURAL = 2,   // dst[(v >> rate) * dst_stride + (i << rate) + (v & (2^rate-1))], i natural, times mul
-                         // and tab_out (one-pass transforms: a tile is a whole virtual column)
+    STORE_NATURAL = 2,   // last pass (S == 1): dst[(v >> rate) * dst_stride + (i << rate) + (v & (2^rate-1))], i
+                         // natural, times mul and tab_out
     STORE_ROWS = 1,      // leaf-major: dst[(rev_rate(v & mask) * n + position) * cols + (v >> rate)]
 };
 
