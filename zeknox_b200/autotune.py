@@ -63,7 +63,7 @@ def leaf_threads(h, lg):
     """CTA sizes of the leaf kernel of hash h for 2^lg leaves, the built-in one first."""
     if h not in MMA_HASHES:
         return [256, 128, 64]
-    first = 32 if lg <= 15 else 128 if h == 4 else 64
+    first = 32 if lg <= 16 else 128 if h == 4 else 64
     return [first] + [t for t in (128, 64, 32) if t != first]
 
 

@@ -532,6 +532,20 @@ __device__ __forceinline__ void mma_set_lane(uint32_t *sm, int kb, int q, uint64
     p[M::ROWS] = (uint32_t)(v >> 32);
 }
 
+// A word of a leaf or node row.  The 32-state form's rows are in global memory
+// and read once, whole sectors at a time: kept out of L1, which the tables fill.
+template <int NS>
+__device__ __forceinline__ uint64_t mma_row_ld(const uint64_t *p)
+{
+    if constexpr (NS == 4) {
+        uint64_t v;
+        asm("ld.global.L1::no_allocate.u64 %0, [%1];" : "=l"(v) : "l"(p));
+        return v;
+    } else {
+        return *p;
+    }
+}
+
 // sponge_hash_one for the warp's states: row(q) is where state q's len words
 // are; the digest word t of state q is left in d[q] (canonical).  len > 4.
 template <int H, int NS, bool TSM = false, class Row>
@@ -548,8 +562,8 @@ __device__ __forceinline__ void sponge_hash_mma(Row row, uint64_t len, uint32_t 
 #pragma unroll
         for (int q = 0; q < NS; q++) {
             const uint64_t *p = row(q) + idx;
-            if (idx + t < len) mma_set_lane<NS>(sm, 0, q, p[t]);
-            if (idx + 4 + t < len) mma_set_lane<NS>(sm, 1, q, p[4 + t]);
+            if (idx + t < len) mma_set_lane<NS>(sm, 0, q, mma_row_ld<NS>(p + t));
+            if (idx + 4 + t < len) mma_set_lane<NS>(sm, 1, q, mma_row_ld<NS>(p + 4 + t));
         }
         // what the next chunk leaves in place: a full one lanes 8..11, one of
         // k < 8 words also lanes k..7

@@ -26,10 +26,10 @@ namespace zk {
 // Default threads per CTA of the leaf kernel ("leaf_threads.<hash>", 32 for
 // the tensor-core hashes only).  Poseidon-BN128's holds 152 registers a
 // thread: three 128-thread CTAs fit an SM where one 256-thread CTA does.  The
-// tensor-core hashes take one-warp CTAs up to 2^15 leaves, where an SM has a
+// tensor-core hashes take one-warp CTAs up to 2^16 leaves, where an SM has a
 // handful of warps and larger CTAs leave some SMs one more than others
-// (Poseidon2 2^15 x 135: 857 against 880 us with 64 threads, 837 at the
-// one-thread-per-leaf form; 2^14: 493 against 509), above that 64 (Poseidon2
+// (Poseidon2 2^15 x 135: 763 against 880 us with 64 threads and 640 a
+// multiprocessor; 2^14: 493 against 509), above that 64 (Poseidon2
 // 2^20 x 135: 14.11 against 14.18 ms) or, for Monolith, 128 (5.14 against 5.30).
 static constexpr int LEAF_T = 256;
 template <int H>
@@ -37,7 +37,7 @@ static uint64_t leaf_t_default(uint64_t n_leaves)
 {
     if (H == HASH_POSEIDON_BN128) return 128;
     if (!HasMma<H>::value) return LEAF_T;
-    return n_leaves <= (1ULL << 15) ? 32 : H == HASH_MONOLITH ? 128 : 64;
+    return n_leaves <= (1ULL << 16) ? 32 : H == HASH_MONOLITH ? 128 : 64;
 }
 // Threads per CTA of the node-parallel level kernel: 128 for Poseidon-BN128
 // (158 registers: three CTAs per SM instead of one), 256 otherwise.  The wide

@@ -224,14 +224,17 @@ __global__ void merkle_level_kernel(uint64_t *__restrict__ digests, MerkleGeom g
 // span being state q of quad g.  Rows past the end repeat the last one and
 // store nothing.
 
-// Threads per SM the register budget of the 32-leaf form aims at: 640 (96
-// registers).  Poseidon2 2^20 x 135: 14.26 ms against 14.44 at 512; 768 and
-// 1024 spill and were slower (an earlier form: 15.2 and 19.8 against 14.9).
-static constexpr int MMA_THREADS_PER_SM = 640;
+// Threads per SM the register budget of the 32-state form aims at: 640 (96
+// registers) where the GPU is full (Poseidon2 2^20 x 135: 14.23 ms against
+// 14.32 at 512; 768 and 1024 spill: 15.2 and 19.8 against 14.9 in an earlier
+// form), 512 (128 registers) for the one-warp CTAs of forests that give an SM a
+// handful of warps, whose S-boxes then overlap further (2^15 x 135: 763
+// against 863 us).
+__host__ __device__ constexpr int mma_threads_per_sm(int t) { return t == 32 ? 512 : 640; }
 
 // Leaf digests (leaf_size > 4: shorter leaves are copied, not hashed).
 template <int H, int NS, int T>
-__global__ void __launch_bounds__(T, NS == 4 ? MMA_THREADS_PER_SM / T : 1)
+__global__ void __launch_bounds__(T, NS == 4 ? mma_threads_per_sm(T) / T : 1)
     merkle_leaf_mma_kernel(const uint64_t *__restrict__ leaves, uint64_t *__restrict__ digests,
                            uint64_t *__restrict__ caps, MerkleGeom g)
 {
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(T, NS == 4 ? MMA_THREADS_PER_SM / T : 1)
 
 // One level of height u, every node of every subtree.
 template <int H, int NS, int T>
-__global__ void __launch_bounds__(T, NS == 4 ? MMA_THREADS_PER_SM / T : 1)
+__global__ void __launch_bounds__(T, NS == 4 ? mma_threads_per_sm(T) / T : 1)
     merkle_level_mma_kernel(uint64_t *__restrict__ digests, MerkleGeom g, uint32_t u)
 {
     __shared__ __align__(16) uint32_t sm[T / 32][MmaSmem<NS>::template words<H>()];
