@@ -13,7 +13,7 @@ import zeknox_b200 as zk
 from zeknox_b200 import autotune
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-KNOBS = {"leaf_threads": {64, 128, 256}, "lde_chunk_mib": None, "lde_last_logr": set(range(1, 9)),
+KNOBS = {"leaf_threads": {32, 64, 128, 256}, "lde_chunk_mib": None, "lde_last_logr": set(range(1, 9)),
          "wide_level_nodes": None, "coop_leaves": None, "lde_host_chunk_mib": None,
          "ntt_split_logr": {0, 7, 8, 9, 10}, "transpose_bulk": set(range(10))}
 
@@ -115,3 +115,66 @@ def test_autotune_candidates_include_the_defaults():
         assert all(v in KNOBS[knob] for v in autotune.CANDIDATES[knob]) if KNOBS[knob] else True
     for lg, cols in autotune.lde_shapes(False):
         assert cols >= 16 and (cols << (lg + autotune.RATE)) <= 1 << 27
+
+
+@pytest.mark.parametrize("quick", [True, False])
+def test_autotune_shapes(quick):
+    for shapes in (autotune.lde_shapes, autotune.ntt_shapes, autotune.transpose_shapes):
+        assert all(lg >= 1 and cols >= 1 for lg, cols in shapes(quick))
+    for h, lg, leaf in autotune.merkle_shapes(quick):
+        threads = autotune.leaf_threads(h, lg)
+        assert h in autotune.HASH_NAMES and leaf > 4 and set(threads) <= KNOBS["leaf_threads"]
+        assert len(set(threads)) == len(threads)
+
+
+@pytest.mark.parametrize("argv", [[], ["--quick"], ["--only", "merkle"]])
+def test_autotune_run_writes_its_table(clean_table, tmp_path, monkeypatch, capsys, argv):
+    """A whole run with the GPU's part faked: every search at every shape, the
+    table, and the closing count."""
+    import torch
+
+    class FakeTimer:
+        def __init__(self, *a):
+            pass
+
+        def on(self, stream):
+            return self
+
+        def __call__(self, fn):  # one candidate of leaf_threads is clearly faster, the rest are even
+            return 0.5 if zk.tune_get("leaf_threads.3", 18) == 128 else 1.0
+
+    def merkle(z, t, timer, h, lg, leaf, margin, log):
+        threads = autotune.leaf_threads(h, lg)
+        args = (lambda: None, lambda k, v: None, margin, log)
+        autotune.search(z, timer, "leaf_threads.%d" % h, lg, threads, threads[0], *args)
+        if (h, lg) == (3, 18):
+            z.tune_set("leaf_threads.3", threads[0], lg=18)  # the other searches at even times
+        for knob in ("wide_level_nodes", "coop_leaves"):
+            autotune.search(z, timer, "%s.%d" % (knob, h), lg, autotune.CANDIDATES[knob], autotune.DEFAULTS[knob], *args)
+
+    def other(*knobs):
+        def tune(z, t, timer, *a):
+            lg, margin, log = a[-4], a[-2], a[-1]
+            for k in knobs:
+                autotune.search(z, timer, k, lg, autotune.CANDIDATES[k], autotune.DEFAULTS[k], lambda: None,
+                                lambda *_: None, margin, log)
+        return tune
+
+    monkeypatch.setenv("ZEKNOX_TUNE_FILE", "none")
+    for name, value in {"is_available": lambda: True, "set_device": lambda d: None, "Stream": lambda: None,
+                        "default_stream": lambda: None, "empty_cache": lambda: None,
+                        "get_device_name": lambda d: "a GPU"}.items():
+        monkeypatch.setattr(torch.cuda, name, value)
+    monkeypatch.setattr(autotune, "Timer", FakeTimer)
+    monkeypatch.setattr(autotune, "tune_merkle", merkle)
+    monkeypatch.setattr(autotune, "tune_lde", other("lde_last_logr", "lde_chunk_mib"))
+    monkeypatch.setattr(autotune, "tune_ntt", other("ntt_split_logr"))
+    monkeypatch.setattr(autotune, "tune_transpose", other("transpose_bulk"))
+    out = tmp_path / "t.txt"
+    autotune.main(argv + ["--out", str(out)])
+    assert capsys.readouterr().out.rstrip().endswith("1 differ from the built-in defaults")
+    zk.tune_clear()
+    zk.tune_load(out)  # what it wrote is a table the library reads
+    assert zk.tune_get("leaf_threads.3", 18) == 128
+    monkeypatch.setattr(zk, "TUNE_TABLE", str(out))
+    test_committed_table_is_well_formed()
