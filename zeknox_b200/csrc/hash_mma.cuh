@@ -80,7 +80,8 @@ __device__ __forceinline__ void mma_16832(uint32_t d[4], uint32_t a0, uint32_t a
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
 }
 
-// s0 + 2^8 s1 + ... + 2^56 s7 (sums below 2^24) as a 64-bit representative.
+// s0 + 2^8 s1 + ... + 2^56 s7 as a 64-bit representative.  257 times the
+// largest sum is below 2^32 (mma_sums_fit, checked when the tables are made).
 __device__ __forceinline__ uint64_t mma_combine(uint32_t s0, uint32_t s1, uint32_t s2, uint32_t s3, uint32_t s4,
                                                 uint32_t s5, uint32_t s6, uint32_t s7)
 {

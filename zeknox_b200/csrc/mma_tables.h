@@ -6,8 +6,9 @@
 //     sum_lanes c x  =  sum_b 2^(8b) sum_(lane, i) x_i * byte_b(c * 2^(8i) mod p),
 // so eight byte columns per output lane hold the reduction of every shifted
 // coefficient already, and an 8-bit tensor-core product with 32-bit sums gives
-// the eight sums exactly (at most 34 lanes * 8 bytes * 255 * 255 < 2^24,
-// checked below for the actual coefficients).
+// the eight sums exactly.  The largest sums any input can reach are 9,092,025
+// (Poseidon), 9,174,390 (Poseidon2) and 41,055 (Monolith), below the
+// 16,711,935 that mma_combine's 32-bit words hold (mma_sums_fit).
 //
 // The 22 partial rounds of Poseidon and Poseidon2 are affine but for the S-box
 // on lane 0, so lane 0 before the S-box of partial round r is an affine form
@@ -43,6 +44,9 @@ struct MmaTables {
     uint64_t h[3] = {};       // coefficients inside a block of partial rounds
     uint64_t worst_sum = 0;   // largest byte-column sum any input can reach
 };
+
+// mma_combine adds 256 times one sum to another in a 32-bit word.
+constexpr bool mma_sums_fit(uint64_t worst_sum) { return 257 * worst_sum < (1ULL << 32); }
 
 namespace mma_gen {
 
@@ -138,6 +142,14 @@ void emit_const(MmaTables &t, F value)
         }
 }
 
+inline void check_sums(const MmaTables &t)
+{
+    if (!mma_sums_fit(t.worst_sum)) {
+        fprintf(stderr, "mma_tables: a byte-column sum can reach %llu\n", (unsigned long long)t.worst_sum);
+        abort();
+    }
+}
+
 inline void expect(const MmaTables &t, size_t words, const char *what)
 {
     if (t.w.size() != words) {
@@ -161,7 +173,7 @@ inline MmaTables make_mma_monolith()
     for (int r = 0; r < 7; r++)
         for (int j = 0; j < 3; j++) emit_const(t, [&](int q) { return rc[12 * r + 4 * j + q]; });
     expect(t, MMA_MONO_WORDS, "end");
-    if (t.worst_sum >= (1ULL << 24)) abort();
+    check_sums(t);
     return t;
 }
 
@@ -233,10 +245,7 @@ inline MmaTables make_mma_tables(int hash)
     for (int b = 0; b < 6; b++)
         emit_const(t, [&](int q) -> uint64_t { return 4 * b + q < 22 ? y[4 * b + q].c : 0; });
     expect(t, MMA_WORDS, "end");
-    if (t.worst_sum >= (1ULL << 24)) {
-        fprintf(stderr, "mma_tables: a byte-column sum can reach %llu\n", (unsigned long long)t.worst_sum);
-        abort();
-    }
+    check_sums(t);
     return t;
 }
 
