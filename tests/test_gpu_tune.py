@@ -84,3 +84,44 @@ def test_batch_graph_rerecorded_after_knob_change():
     assert np.array_equal(to_np(leaves), rows)
     assert np.array_equal(to_np(caps).reshape(-1, 4), cp)
     assert np.array_equal(to_np(dig).reshape(-1, 4), d)
+
+
+def test_transforms_while_another_thread_sets_knobs():
+    """Knobs that change the number of passes and the chunk, set and cleared by
+    another thread: every call plans its temporaries and its launches alike."""
+    import threading
+
+    stop = threading.Event()
+
+    def turn():
+        k = 0
+        while not stop.is_set():
+            k += 1
+            zk.tune_set("ntt_split_logr", (0, 7, 8)[k % 3])
+            zk.tune_set("lde_last_logr", (8, 3)[k % 2])
+            zk.tune_set("lde_chunk_mib", (512, 1)[k % 2])
+            if k % 5 == 0:
+                zk.tune_clear()
+
+    lg, rate, cols = 12, 1, 33
+    c = O.field_data(5, cols << lg)
+    want = (O.batched_ntt(c, lg, cols), O.batched_lde(c, lg, rate, cols), O.lde_rows(c, lg, rate, cols),
+            O.lde_rows(c[:cols << 8], 8, rate, cols))
+    ext = torch.zeros(cols << (lg + rate), dtype=torch.int64, device="cuda")
+    inp = to_dev(c)
+    t = threading.Thread(target=turn)
+    t.start()
+    try:
+        for _ in range(60):
+            x = inp.clone()
+            zk.ntt_batch(0, x, lg, cols)
+            assert np.array_equal(to_np(x), want[0])
+            zk.lde_batch(0, ext, inp, lg, cols, rate)
+            assert np.array_equal(to_np(ext), want[1])
+            zk.lde_rows(0, ext, inp, lg, rate, cols)
+            assert np.array_equal(to_np(ext), want[2])
+            zk.lde_rows(0, ext, inp, 8, rate, cols)  # one pass at radix 2^8, several below
+            assert np.array_equal(to_np(ext)[:cols << (8 + rate)], want[3])
+    finally:
+        stop.set()
+        t.join()

@@ -51,6 +51,7 @@ template <class F>
 RustError guarded(F &&f)
 {
     try {
+        zk::TunePin pin;
         f();
         return ok();
     } catch (const zk::arg_failure &e) {
@@ -103,9 +104,11 @@ void on_each_gpu(uint32_t gpus, F &&fn)
     }
     std::vector<std::exception_ptr> errs(gpus);
     std::vector<std::thread> threads;
+    const zk::TuneVersion knobs = zk::tune_version();
     for (uint32_t g = 0; g < gpus; g++)
         threads.emplace_back([&, g] {
             try {
+                zk::TunePin pin(knobs);
                 fn(g);
             } catch (...) {
                 errs[g] = std::current_exception();

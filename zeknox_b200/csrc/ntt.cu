@@ -170,6 +170,7 @@ static void run_dif(DeviceCtx &c, const DifJob &j)
         throw arg_failure("zero-size transform");
     }
     auto passes = plan_passes(j.L, j.rows);
+    if (passes.size() > 1 && !(j.rows ? j.scratch : j.dst)) throw arg_failure("null scratch of a transform of several passes");
     const uint64_t n = 1ULL << j.L;
     const uint64_t *tw_small = c.twiddles(12, j.inverse);
     for (size_t pi = 0; pi < passes.size(); pi++) {
@@ -268,7 +269,8 @@ static void reorder(DeviceCtx &c, const uint64_t *src, uint64_t src_stride, uint
     ZK_CUDA(cudaGetLastError());
 }
 
-// Whether column transforms of 2^L points take one pass.
+// Whether column transforms of 2^L points take one pass (the callers hold a
+// TunePin, so run_dif plans the same).
 static bool one_pass(uint32_t L) { return plan_passes(L, false).size() == 1; }
 
 // --------------------------------------------------------------- public ops

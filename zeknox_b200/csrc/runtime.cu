@@ -36,11 +36,25 @@ static std::atomic<uint64_t> g_launches{0};
 void note_launch(uint64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 uint64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
-static std::mutex g_tune_mu;
-static std::map<std::pair<std::string, uint32_t>, uint64_t> g_tune;
-static std::atomic<uint64_t> g_tune_gen{0};
+struct TuneTable {
+    std::map<std::pair<std::string, uint32_t>, uint64_t> knobs;
+    uint64_t generation = 0;
+};
 
-uint64_t tune_generation() { return g_tune_gen.load(std::memory_order_relaxed); }
+static std::mutex g_tune_mu;
+static TuneVersion g_tune = std::make_shared<const TuneTable>();  // the newest
+static thread_local TuneVersion t_pinned;
+
+// The newest table with `change` made to it becomes the newest.
+template <class F>
+static void tune_update(F &&change)
+{
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto next = std::make_shared<TuneTable>(*g_tune);
+    change(next->knobs);
+    next->generation++;
+    g_tune = std::move(next);
+}
 
 // A table named by ZEKNOX_TUNE_FILE ("none": no table) is read at the first
 // knob lookup, so consumers of the C ABI get tuned knobs without calling
@@ -57,28 +71,36 @@ static void tune_env_load()
     }
 }
 
-uint64_t tune_get(const std::string &name, uint32_t lg, uint64_t dflt)
+TuneVersion tune_version()
 {
+    if (t_pinned) return t_pinned;
     std::call_once(g_tune_env_once, tune_env_load);
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    auto it = g_tune.find({name, lg});
-    if (it != g_tune.end()) return it->second;
-    it = g_tune.find({name, TUNE_ANY});
-    return it != g_tune.end() ? it->second : dflt;
+    return g_tune;
+}
+
+TunePin::TunePin(TuneVersion v) : keep_(std::move(v)), before_(std::move(t_pinned)) { t_pinned = keep_; }
+TunePin::~TunePin() { t_pinned = std::move(before_); }
+
+uint64_t tune_generation() { return tune_version()->generation; }
+
+uint64_t tune_get(const std::string &name, uint32_t lg, uint64_t dflt)
+{
+    const TuneVersion v = tune_version();
+    auto it = v->knobs.find({name, lg});
+    if (it != v->knobs.end()) return it->second;
+    it = v->knobs.find({name, TUNE_ANY});
+    return it != v->knobs.end() ? it->second : dflt;
 }
 
 void tune_set(const std::string &name, uint32_t lg, uint64_t value)
 {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[{name, lg}] = value;
-    g_tune_gen.fetch_add(1, std::memory_order_relaxed);
+    tune_update([&](auto &knobs) { knobs[{name, lg}] = value; });
 }
 
 void tune_clear()
 {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune.clear();
-    g_tune_gen.fetch_add(1, std::memory_order_relaxed);
+    tune_update([](auto &knobs) { knobs.clear(); });
 }
 
 void tune_load_file(const char *path)
@@ -107,7 +129,9 @@ void tune_load_file(const char *path)
     }
     fclose(f);
     // all or nothing: a malformed table changes no knob
-    for (auto &e : entries) tune_set(std::get<0>(e), std::get<1>(e), std::get<2>(e));
+    tune_update([&](auto &knobs) {
+        for (auto &e : entries) knobs[{std::get<0>(e), std::get<1>(e)}] = std::get<2>(e);
+    });
 }
 
 static std::mutex g_reg_mu;

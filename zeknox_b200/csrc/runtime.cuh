@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include <map>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -115,10 +116,32 @@ void tune_clear();
 // Reads "<name> <lg|*> <value>" lines ('#' comments); throws arg_failure on a
 // malformed line, in which case no knob is changed.
 void tune_load_file(const char *path);
-// Bumped by every tune_set / tune_clear: cached CUDA graphs record it in their
-// key, so a graph captured under other knob values is not replayed.
+// Number of the table's version, one more with every tune_set, tune_clear and
+// table load: cached CUDA graphs record it in their key, so a graph captured
+// under other knob values is not replayed.
 uint64_t tune_generation();
 constexpr uint32_t TUNE_ANY = 0xFFFFFFFFu;
+
+// The table changes by whole versions, and a call keeps to one: a knob that
+// sizes a temporary is read again for the launches that use it, and another
+// thread may set knobs in between.  While a TunePin lives, tune_get and
+// tune_generation on its thread read the pin's version (without one: that of
+// an enclosing pin, else the newest).  Every entry point that launches holds
+// one; a queued request keeps the version that sized its memory.
+struct TuneTable;
+using TuneVersion = std::shared_ptr<const TuneTable>;
+TuneVersion tune_version();
+class TunePin {
+public:
+    TunePin() : TunePin(tune_version()) {}
+    explicit TunePin(TuneVersion v);
+    ~TunePin();
+    TunePin(const TunePin &) = delete;
+    TunePin &operator=(const TunePin &) = delete;
+
+private:
+    TuneVersion keep_, before_;
+};
 
 // NVTX range over a host-side stage (queuing an LDE, a forest, a commit, a
 // batch): a profiler that records NVTX (nsys, ncu's NVTX filters) shows the

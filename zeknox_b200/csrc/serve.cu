@@ -103,6 +103,7 @@ struct RangeAlloc {
 
 struct Ticket {
     zk_serve_request req;
+    TuneVersion knobs;         // the tuning table that sized the job
     Clock::time_point t_submit, t_admit, t_done;
     int status = 0;  // 0 queued, 1 running, 2 done, < 0 failed or cancelled
     int slot = -1;
@@ -161,6 +162,7 @@ struct Server {
 
     void place(Ticket &t)
     {
+        TunePin pin(t.knobs);
         const zk_serve_request &r = t.req;
         const uint64_t N = 1ULL << (r.lg_n + r.rate_bits);
         const uint64_t n_caps = 1ULL << r.cap_height;
@@ -199,6 +201,7 @@ struct Server {
         cudaStream_t s = slot_stream[slot];
         const uint64_t n_caps = 1ULL << r.cap_height;
         NvtxRange range("zeknox serve start");
+        TunePin pin(t.knobs);
         std::lock_guard<std::recursive_mutex> lk(ctx->mu);
         try {
             zk_commit_job j{};
@@ -406,6 +409,7 @@ struct Server {
     {
         const zk_serve_request &r = t.req;
         NvtxRange range("zeknox serve post");
+        TunePin pin(t.knobs);
         std::lock_guard<std::recursive_mutex> lk(ctx->mu);
         try {
             const uint64_t N = 1ULL << (r.lg_n + r.rate_bits);
@@ -747,6 +751,7 @@ template <class F>
 RustError guard(F &&f)
 {
     try {
+        TunePin pin;
         f();
         return RustError{0, nullptr};
     } catch (const arg_failure &e) {
@@ -896,6 +901,7 @@ extern "C" RustError zeknox_server_submit(void *server, const zk_serve_request *
         const uint64_t id = s->next_id++;
         zk::Ticket &t = s->tickets[id];
         t.req = *req;
+        t.knobs = zk::tune_version();  // this call's pin: job_bytes read it too
         t.bytes = bytes;
         t.t_submit = zk::Clock::now();
         s->queue.push_back(id);
