@@ -568,8 +568,9 @@ static __global__ void __launch_bounds__(256)
         const uint64_t t = blockIdx.x + k * gridDim.x;
         if (t >= n_tiles) return;
         const uint32_t s = (uint32_t)(k % STAGES);
-        const uint64_t i0 = (VEC == 1 ? t / blocks : t % tiles_i) * TI, b0 = (VEC == 1 ? t % blocks : t / tiles_i) * tb;
-        const uint32_t nb = (uint32_t)(cols - b0 < tb ? cols - b0 : tb);
+        const uint32_t width = VEC == 1 ? tb : TB;
+        const uint64_t i0 = (VEC == 1 ? t / blocks : t % tiles_i) * TI, b0 = (VEC == 1 ? t % blocks : t / tiles_i) * width;
+        const uint32_t nb = (uint32_t)(cols - b0 < width ? cols - b0 : width);
         const uint32_t bar = smem_u32(&full[s]);
         if (lane == 0) mbar_arrive_expect_tx(bar, nb * TI * 8 + (k == 0 && blockIdx.x == 0 ? extra_tx : 0));
         __syncwarp();
@@ -593,10 +594,11 @@ static __global__ void __launch_bounds__(256)
             failed = true;
             break;
         }
-        const uint64_t i0 = (VEC == 1 ? t / blocks : t % tiles_i) * TI, b0 = (VEC == 1 ? t % blocks : t / tiles_i) * tb;
+        const uint64_t i0 = (VEC == 1 ? t / blocks : t % tiles_i) * TI;
+        const uint64_t b0 = VEC == 1 ? t % blocks * tb : t / tiles_i * TB;
         const uint64_t *tile = stage_buf + s * STAGE_WORDS;
-        const uint32_t nb = (uint32_t)(cols - b0 < tb ? cols - b0 : tb);
         if constexpr (VEC == 1) {
+            const uint32_t nb = (uint32_t)(cols - b0 < tb ? cols - b0 : tb);
             // warps take whole runs of 2 rows: the row's columns, 16 at a time
             const uint32_t c0 = (lane & 7) + ((lane >> 4) << 3), r0 = (lane >> 3) & 1;
 #pragma unroll 2
@@ -614,8 +616,8 @@ static __global__ void __launch_bounds__(256)
             const uint32_t r = 4 * (w / (TB / 16)) + (l >> 3), c = 2 * (8 * (w % (TB / 16)) + (l & 7));
             const uint64_t b = b0 + c;
             const uint64_t oi = bitrev64(i0 + r, lg) * cols + b;
-            // c even and nb even: c + 1 < nb too
-            if (c < nb && ZK_IN_BOUNDS(oi + 1, n * cols, OOB_TRANSPOSE_OUT)) {
+            // b and cols even: b + 1 < cols too
+            if (b < cols && ZK_IN_BOUNDS(oi + 1, n * cols, OOB_TRANSPOSE_OUT)) {
                 ulonglong2 v;
                 v.x = tile[c * PITCH + r];
                 v.y = tile[(c + 1) * PITCH + r];
