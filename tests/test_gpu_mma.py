@@ -56,3 +56,43 @@ def test_forests_on_every_form(name, states_per_warp):
         zk.tune_clear()
         if zk.os.path.exists(zk.TUNE_TABLE):
             zk.tune_load(zk.TUNE_TABLE)
+
+
+@pytest.mark.parametrize("threads", [32, 64, 128])
+@pytest.mark.parametrize("states_per_warp", [8, 16, 32])
+@pytest.mark.parametrize("name", ["poseidon", "poseidon2", "monolith"])
+def test_forests_with_every_block_size(name, states_per_warp, threads):
+    """Every number of leaves per warp in blocks of one, two and four warps (each
+    its own register budget and shared-memory slices): a block not full, one
+    full, several."""
+    h = HASHES[name]
+    zk.tune_set("leaf_threads.%d" % h, threads)
+    try:
+        for nl, ls, ch in [(2, 9, 0), (32, 12, 1), (128, 20, 2), (512, 17, 3), (2048, 8, 0)]:
+            zk.tune_set("coop_leaves.%d" % h, {8: nl, 16: (nl + 3) // 4, 32: 0}[states_per_warp])
+            leaves = O.field_data(nl * 77 + ls, nl * ls) if ls != 8 else _pick(CANON, nl * ls, nl + threads)
+            dig, cap = run_gpu(leaves, nl, ls, ch, h)
+            d2, c2 = O.merkle(leaves, ls, ch, h)
+            assert np.array_equal(cap, c2), (nl, ls, ch)
+            assert np.array_equal(dig, d2), (nl, ls, ch)
+    finally:
+        zk.tune_clear()
+        if zk.os.path.exists(zk.TUNE_TABLE):
+            zk.tune_load(zk.TUNE_TABLE)
+
+
+@pytest.mark.parametrize("name,lg", [("poseidon", 17), ("poseidon2", 17), ("monolith", 17), ("monolith", 18)])
+def test_large_forests_as_built_in(name, lg):
+    """The forms chosen above 2^16 leaves: 32 per warp in blocks of two warps,
+    Monolith's 16 and 32 per warp in blocks of four."""
+    h, nl, ls = HASHES[name], 1 << lg, 9
+    zk.tune_clear()
+    try:
+        leaves = O.field_data(lg + h, nl * ls)
+        dig, cap = run_gpu(leaves, nl, ls, 4, h)
+    finally:
+        if zk.os.path.exists(zk.TUNE_TABLE):
+            zk.tune_load(zk.TUNE_TABLE)
+    d2, c2 = O.merkle(leaves, ls, 4, h)
+    assert np.array_equal(cap, c2)
+    assert np.array_equal(dig, d2)
