@@ -63,7 +63,8 @@ void prepare_job(DeviceCtx &c, const zk_commit_job &j)
     prepare_tables(c, j.lg_n, j.rate_bits, gen_of(j), j.input_is_values != 0);
 }
 
-void commit_enqueue(DeviceCtx &c, const zk_commit_job &j, cudaStream_t s, uint64_t *scratch, bool host_input)
+void commit_enqueue(DeviceCtx &c, const zk_commit_job &j, cudaStream_t s, uint64_t *scratch, bool host_input,
+                    uint64_t at_once)
 {
     NvtxRange range("zeknox commit");
     const uint64_t n = 1ULL << j.lg_n;
@@ -89,7 +90,7 @@ void commit_enqueue(DeviceCtx &c, const zk_commit_job &j, cudaStream_t s, uint64
         std::string err;
         const uint64_t n_caps = 1ULL << j.cap_height;
         if (!merkle_device(j.digests, j.caps, j.leaves, 2 * (N - n_caps), n_caps, N, j.cols, j.cap_height,
-                           j.hash_type, s, err))
+                           j.hash_type, s, err, at_once))
             throw arg_failure(err);
     } catch (...) {
         c.stream = keep;
@@ -230,22 +231,33 @@ static void run_graph(DeviceCtx &c, std::vector<uint64_t> key, uint32_t njobs, c
     ZK_CUDA(cudaGraphLaunch(g.exec, c.stream));
 }
 
+// Leaves that njobs forests of `total` leaves hash at the same time: those of
+// as many jobs as there are branches.
+static uint64_t leaves_at_once(uint64_t total, uint32_t njobs)
+{
+    return njobs > (uint32_t)BRANCHES ? total / njobs * BRANCHES : total;
+}
+
 void commit_batch_graph(DeviceCtx &c, const zk_commit_job *jobs, uint32_t njobs)
 {
     NvtxRange range("zeknox commit_batch");
     if (njobs == 0) return;
     std::vector<double> cost(njobs);
     std::vector<uint64_t> words(njobs);
+    uint64_t leaves = 0;
     for (uint32_t i = 0; i < njobs; i++) {
         const zk_commit_job &j = jobs[i];
+        leaves += 1ULL << (j.lg_n + j.rate_bits);
         cost[i] = (double)(1ULL << (j.lg_n + j.rate_bits)) * ((j.cols + 7) / 8 + 1);
         if (is_host_pointer(j.input)) throw arg_failure("batched commits take device inputs");
         words[i] = commit_scratch_words(j.lg_n, j.rate_bits, j.cols, j.input_is_values != 0, false);
         prepare_job(c, j);
     }
     ZK_CUDA(cudaStreamSynchronize(c.stream));
-    run_graph(c, batch_key(jobs, njobs), njobs, cost, words,
-              [&](uint32_t i, cudaStream_t s, uint64_t *scratch) { commit_enqueue(c, jobs[i], s, scratch); });
+    const uint64_t at_once = leaves_at_once(leaves, njobs);
+    run_graph(c, batch_key(jobs, njobs), njobs, cost, words, [&](uint32_t i, cudaStream_t s, uint64_t *scratch) {
+        commit_enqueue(c, jobs[i], s, scratch, false, at_once);
+    });
 }
 
 void merkle_batch_graph(DeviceCtx &c, const zk_merkle_job *jobs, uint32_t njobs)
@@ -257,6 +269,7 @@ void merkle_batch_graph(DeviceCtx &c, const zk_merkle_job *jobs, uint32_t njobs)
     std::vector<uint64_t> key;
     key.push_back(0xFEEDULL);  // distinct from commit keys
     key.push_back(tune_generation());
+    uint64_t leaves = 0;
     for (uint32_t i = 0; i < njobs; i++) {
         const zk_merkle_job &j = jobs[i];
         std::string err;
@@ -265,17 +278,19 @@ void merkle_batch_graph(DeviceCtx &c, const zk_merkle_job *jobs, uint32_t njobs)
             throw arg_failure("tree " + std::to_string(i) + ": " + (err.empty() ? "bad cap_height" : err));
         if (j.hash_type > 4) throw arg_failure("tree " + std::to_string(i) + ": unsupported hash_type");
         if (!j.leaves || !j.caps || (!j.digests && n_caps < j.n_leaves)) throw arg_failure("null buffer");
+        leaves += j.n_leaves;
         cost[i] = (double)j.n_leaves * ((j.leaf_size + 7) / 8 + 1);
         for (uint64_t v : {(uint64_t)j.leaves, (uint64_t)j.digests, (uint64_t)j.caps, j.n_leaves, j.leaf_size,
                            ((uint64_t)j.cap_height << 32) | j.hash_type})
             key.push_back(v);
     }
+    const uint64_t at_once = leaves_at_once(leaves, njobs);
     run_graph(c, std::move(key), njobs, cost, words, [&](uint32_t i, cudaStream_t s, uint64_t *) {
         const zk_merkle_job &j = jobs[i];
         std::string err;
         const uint64_t n_caps = 1ULL << j.cap_height;
         if (!merkle_device(j.digests, j.caps, j.leaves, 2 * (j.n_leaves - n_caps), n_caps, j.n_leaves, j.leaf_size,
-                           j.cap_height, j.hash_type, s, err))
+                           j.cap_height, j.hash_type, s, err, at_once))
             throw arg_failure(err);
     });
 }

@@ -24,7 +24,9 @@ bool device_can_read(const void *p, int dev);
 // null when that is 0).  Allocates nothing and never synchronises, so it can be
 // recorded into a CUDA graph once prepare_job() has built the tables it reads.
 // host_input: j.input is host memory, staged through the scratch chunk by chunk.
-void commit_enqueue(DeviceCtx &c, const zk_commit_job &j, cudaStream_t s, uint64_t *scratch, bool host_input = false);
+// at_once: leaves of all forests queued to run at the same time (0: this one alone).
+void commit_enqueue(DeviceCtx &c, const zk_commit_job &j, cudaStream_t s, uint64_t *scratch, bool host_input = false,
+                    uint64_t at_once = 0);
 void prepare_job(DeviceCtx &c, const zk_commit_job &j);
 
 // Run a batch of commits: the launches of every job are recorded once into a

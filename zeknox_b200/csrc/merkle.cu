@@ -66,6 +66,13 @@ constexpr uint64_t mid_leaves()
 static constexpr uint64_t WIDE_LEVEL_NODES = 1ULL << 15;  // default: levels at least this wide run node-parallel
                                                           // ("wide_level_nodes.<hash>")
 
+// A level of a forest beside others counts their nodes too from this many of
+// its own on (one batch of forests; not at all / from 1 / 2^9 / 2^11 / 2^13
+// nodes, us, Poseidon2): 8 of 2^13 x 9 492 / 379 / 375 / 376 / 490; 2 of 2^18 and
+// 14 of 2^9..2^12 x 8 1203 / 1419 / 1258 / 1161 / 1204; 64 of 2^10..2^16 x 8 5027 /
+// 4062 / 3994 / 3943 / 4030; Poseidon alike, Monolith by less.
+static constexpr uint64_t BESIDE_NODES = 1ULL << 11;
+
 // Poseidon-BN128 forests up to this many leaves hash them with five threads a
 // state ("coop_leaves.2"): 2^12 x 135 7.2 against 11.0 ms with one, 2^13 9.6
 // against 11.2, 2^14 13.7 against 11.3.
@@ -127,8 +134,18 @@ static void launch_level(uint64_t total, uint64_t *digests, const MerkleGeom &g,
     note_launch();
 }
 
+// at_once: leaves of all forests that run at the same time, this one's among
+// them.  Several forests' narrow levels fill the GPU together, where the
+// fold's latency form (8 nodes per warp) costs more than one launch per level
+// saves: a level is wide when the forests have wide_level_nodes nodes at its
+// height between them.  Batches of Poseidon2 commits, each forest by its own
+// width / by all of them (us): 7 of 2^13..2^15 leaves x 5..16 827 / 604, 9 of
+// 2^12..2^16 x 8..20 1286 / 994.  The leaf kernel's form and the fold's
+// table copy stay with the forest's own size: by all leaves the forms came out
+// within 1% in the mean, and without the copy batches took 2% longer.
 template <int H>
-static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *leaves, const MerkleGeom &g, cudaStream_t s)
+static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *leaves, const MerkleGeom &g, uint64_t at_once,
+                          cudaStream_t s)
 {
     const uint32_t lg_leaves = ilog2_exact(g.n_leaves);
     const uint64_t lt = tune_get("leaf_threads." + std::to_string(H), lg_leaves, leaf_t_default<H>(g.n_leaves));
@@ -163,7 +180,11 @@ static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *lea
     if (g.sub_leaves == 1) return;  // caps == leaves
     // Wide levels: one node per thread while a level still fills the GPU.
     const uint32_t top = g.log_sub - 1;
-    while (u0 + 1 <= top && (g.n_leaves >> (u0 + 1)) >= wide) {
+    const auto wide_level = [&](uint32_t u) {
+        const uint64_t nodes = g.n_leaves >> u;
+        return nodes >= wide || (HasMma<H>::value && nodes >= BESIDE_NODES && (at_once >> u) >= wide);
+    };
+    while (u0 + 1 <= top && wide_level(u0 + 1)) {
         u0++;
         const uint64_t total = g.n_leaves >> u0;
         launch_level<H>(total, digests, g, u0, s);
@@ -202,7 +223,7 @@ static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *lea
 
 bool merkle_device(uint64_t *digests, uint64_t *caps, const uint64_t *leaves, uint64_t n_digests, uint64_t n_caps,
                    uint64_t n_leaves, uint64_t leaf_size, uint64_t cap_height, uint64_t hash_type, cudaStream_t stream,
-                   std::string &err)
+                   std::string &err, uint64_t at_once)
 {
     NvtxRange range("zeknox merkle");
     if (!merkle_geometry_ok(n_digests, n_caps, n_leaves, cap_height, err)) return false;
@@ -218,11 +239,11 @@ bool merkle_device(uint64_t *digests, uint64_t *caps, const uint64_t *leaves, ui
     g.log_sub = ilog2_exact(g.sub_leaves);
     g.n_caps = (uint32_t)n_caps;
     switch (hash_type) {
-    case HASH_POSEIDON: merkle_launch<HASH_POSEIDON>(digests, caps, leaves, g, stream); break;
-    case HASH_KECCAK: merkle_launch<HASH_KECCAK>(digests, caps, leaves, g, stream); break;
-    case HASH_POSEIDON_BN128: merkle_launch<HASH_POSEIDON_BN128>(digests, caps, leaves, g, stream); break;
-    case HASH_POSEIDON2: merkle_launch<HASH_POSEIDON2>(digests, caps, leaves, g, stream); break;
-    case HASH_MONOLITH: merkle_launch<HASH_MONOLITH>(digests, caps, leaves, g, stream); break;
+    case HASH_POSEIDON: merkle_launch<HASH_POSEIDON>(digests, caps, leaves, g, at_once, stream); break;
+    case HASH_KECCAK: merkle_launch<HASH_KECCAK>(digests, caps, leaves, g, at_once, stream); break;
+    case HASH_POSEIDON_BN128: merkle_launch<HASH_POSEIDON_BN128>(digests, caps, leaves, g, at_once, stream); break;
+    case HASH_POSEIDON2: merkle_launch<HASH_POSEIDON2>(digests, caps, leaves, g, at_once, stream); break;
+    case HASH_MONOLITH: merkle_launch<HASH_MONOLITH>(digests, caps, leaves, g, at_once, stream); break;
     default:
         err = "unsupported hash_type " + std::to_string(hash_type);
         return false;

@@ -94,10 +94,11 @@ void transpose_rev_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint3
 void salt_device(DeviceCtx &c, uint64_t *out, uint64_t count);
 
 // Merkle forest on device memory, launched on `stream`; returns false (with a
-// message in err) on invalid geometry or an unsupported hash.
+// message in err) on invalid geometry or an unsupported hash.  at_once: leaves
+// of all forests queued to run at the same time (0: this one alone).
 bool merkle_device(uint64_t *digests, uint64_t *caps, const uint64_t *leaves, uint64_t n_digests, uint64_t n_caps,
                    uint64_t n_leaves, uint64_t leaf_size, uint64_t cap_height, uint64_t hash_type, cudaStream_t stream,
-                   std::string &err);
+                   std::string &err, uint64_t at_once = 0);
 
 bool merkle_geometry_ok(uint64_t n_digests, uint64_t n_caps, uint64_t n_leaves, uint64_t cap_height, std::string &err);
 
