@@ -2,8 +2,9 @@
 //
 // Semantics follow zeknox native/ntt/ntt.cu (batch_ntt :253-309, batch_lde
 // :477-564, compute_transpose_rev :182-226); the execution plan is this
-// project's: a handful of multi-stage DIF passes (ntt.cuh) plus one tiled
-// reorder, instead of one HBM pass per radix-2 stage.
+// project's: a handful of multi-stage DIF passes (ntt.cuh), the last of which
+// writes natural order or bit-reversed leaf rows itself, instead of one HBM pass
+// per radix-2 stage.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -126,8 +127,8 @@ static std::vector<Pass> plan_passes_last(uint32_t L, bool rows, uint32_t last_r
 // The last pass of a row-output transform has radix 2^lde_last_logr (tuned).
 static std::vector<Pass> plan_passes(uint32_t L, bool rows)
 {
-    return plan_passes_last(L, rows, (uint32_t)tune_get("lde_last_logr", L, MAX_ROWS_LOGR),
-                            rows ? 0 : (uint32_t)tune_get("ntt_split_logr", L, 0));
+    return rows ? plan_passes_last(L, true, (uint32_t)tune_get("lde_last_logr", L, MAX_ROWS_LOGR))
+                : plan_passes_last(L, false, MAX_ROWS_LOGR, (uint32_t)tune_get("ntt_split_logr", L, 0));
 }
 
 // Batched DIF over `vcols` virtual columns of size 2^L; output in bit-reversed
@@ -135,6 +136,7 @@ static std::vector<Pass> plan_passes(uint32_t L, bool rows)
 // rows=true, as leaf rows (see STORE_ROWS).  `scratch` (vcols * 2^L words) is
 // needed only when rows=true and there is more than one pass.
 struct DifJob {
+    const std::vector<Pass> *passes;  // planned once per call: the temporaries are sized by them too
     const uint64_t *src;
     uint64_t src_stride;
     int load;                 // NttLoad of the first pass
@@ -169,7 +171,7 @@ static void run_dif(DeviceCtx &c, const DifJob &j)
         // size-1 transform: copy (with scaling) -- handled by the caller's reorder
         throw arg_failure("zero-size transform");
     }
-    auto passes = plan_passes(j.L, j.rows);
+    const std::vector<Pass> &passes = *j.passes;
     if (passes.size() > 1 && !(j.rows ? j.scratch : j.dst)) throw arg_failure("null scratch of a transform of several passes");
     const uint64_t n = 1ULL << j.L;
     const uint64_t *tw_small = c.twiddles(12, j.inverse);
@@ -269,10 +271,6 @@ static void reorder(DeviceCtx &c, const uint64_t *src, uint64_t src_stride, uint
     ZK_CUDA(cudaGetLastError());
 }
 
-// Whether column transforms of 2^L points take one pass (the callers hold a
-// TunePin, so run_dif plans the same).
-static bool one_pass(uint32_t L) { return plan_passes(L, false).size() == 1; }
-
 // --------------------------------------------------------------- public ops
 
 void ntt_batch_device(DeviceCtx &c, uint64_t *inout, uint32_t lg, uint64_t batches, bool inverse, bool with_coset,
@@ -297,8 +295,10 @@ void ntt_batch_device(DeviceCtx &c, uint64_t *inout, uint32_t lg, uint64_t batch
     // reference order: coset multiply (forward powers) then n^-1 (ntt.cu:137-143)
     j.mul = inverse ? H_SIZE_INV[lg] : 1;
     j.tab_out = inverse ? coset : nullptr;
+    const auto passes = plan_passes(lg, false);
+    j.passes = &passes;
     DevBuf tmp;
-    if (!scratch && !one_pass(lg)) {
+    if (!scratch && passes.size() > 1) {
         tmp.ctx = &c;
         scratch = tmp.p = c.alloc(n * batches * 8);
     }
@@ -342,8 +342,10 @@ void lde_batch_device(DeviceCtx &c, uint64_t *out, const uint64_t *in, uint32_t 
     j.dst_stride = 1ULL << j.L;
     j.out = out;
     j.out_stride = N;
+    const auto passes = plan_passes(j.L, false);
+    j.passes = &passes;
     DevBuf tmp;
-    if (!one_pass(j.L)) {
+    if (passes.size() > 1) {
         tmp.ctx = &c;
         j.dst = tmp.p = c.alloc(N * batches * 8);
     } else if (in < out + N * batches && out < in + n * batches) {
@@ -586,7 +588,8 @@ void lde_rows_device(DeviceCtx &c, uint64_t *rows, const uint64_t *coeffs, uint3
     NvtxRange range("zeknox lde_rows");
     const uint64_t n = 1ULL << lg_n;
     if (cols == 0) return;
-    const bool multi = plan_passes(lg_n, true).size() > 1;
+    const auto passes = plan_passes(lg_n, true);
+    const bool multi = passes.size() > 1;
     uint64_t chunk = multi ? lde_rows_chunk_cols(lg_n, rate, cols) : cols;
     if (multi && host_coeffs) {
         // never above the scratch sized by lde_rows_chunk_cols
@@ -620,6 +623,7 @@ void lde_rows_device(DeviceCtx &c, uint64_t *rows, const uint64_t *coeffs, uint3
         const uint64_t cc = cols - c0 < chunk ? cols - c0 : chunk;
         if (host_coeffs) ZK_CUDA(cudaStreamWaitEvent(c.stream, c.chunk_event(k), 0));
         DifJob j{};
+        j.passes = &passes;
         j.src = coeffs + c0 * n;
         j.src_stride = n;
         j.load = LOAD_COSETS;

@@ -43,7 +43,7 @@ struct TuneTable {
 
 static std::mutex g_tune_mu;
 static TuneVersion g_tune = std::make_shared<const TuneTable>();  // the newest
-static thread_local TuneVersion t_pinned;
+static thread_local const TuneVersion *t_pinned = nullptr;  // the innermost pin's
 
 // The newest table with `change` made to it becomes the newest.
 template <class F>
@@ -73,24 +73,26 @@ static void tune_env_load()
 
 TuneVersion tune_version()
 {
-    if (t_pinned) return t_pinned;
+    if (t_pinned) return *t_pinned;
     std::call_once(g_tune_env_once, tune_env_load);
     std::lock_guard<std::mutex> lk(g_tune_mu);
     return g_tune;
 }
 
-TunePin::TunePin(TuneVersion v) : keep_(std::move(v)), before_(std::move(t_pinned)) { t_pinned = keep_; }
-TunePin::~TunePin() { t_pinned = std::move(before_); }
+TunePin::TunePin(TuneVersion v) : keep_(std::move(v)), before_(t_pinned) { t_pinned = &keep_; }
+TunePin::~TunePin() { t_pinned = before_; }
 
 uint64_t tune_generation() { return tune_version()->generation; }
 
 uint64_t tune_get(const std::string &name, uint32_t lg, uint64_t dflt)
 {
-    const TuneVersion v = tune_version();
-    auto it = v->knobs.find({name, lg});
-    if (it != v->knobs.end()) return it->second;
-    it = v->knobs.find({name, TUNE_ANY});
-    return it != v->knobs.end() ? it->second : dflt;
+    TuneVersion newest;
+    if (!t_pinned) newest = tune_version();
+    const auto &knobs = (t_pinned ? *t_pinned : newest)->knobs;
+    auto it = knobs.find({name, lg});
+    if (it != knobs.end()) return it->second;
+    it = knobs.find({name, TUNE_ANY});
+    return it != knobs.end() ? it->second : dflt;
 }
 
 void tune_set(const std::string &name, uint32_t lg, uint64_t value)

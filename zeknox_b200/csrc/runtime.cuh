@@ -105,7 +105,7 @@ uint32_t ilog2_exact(uint64_t x);  // -1u if x is not a power of two
 
 // Tuning table: named knobs, optionally per log2 size, set by the autotuner
 // (zeknox_tune_set / zeknox_tune_load); tune_get falls back to the size-free
-// entry and then to `dflt`.  Knobs: "leaf_threads.<hash>" (64/128/256; 32 for the tensor-core hashes),
+// entry and then to `dflt`.  Knobs: "leaf_threads.<hash>" (64/128/256; 32/64/128 for the tensor-core hashes),
 // "lde_chunk_mib", "lde_host_chunk_mib", "lde_last_logr" (1..8), "wide_level_nodes.<hash>",
 // "coop_leaves.<hash>", "transpose_bulk" (0 16-byte form, 1..8 bulk-copy tile
 // shape, 9 by column count), "ntt_split_logr" (largest pass of a
@@ -140,7 +140,8 @@ public:
     TunePin &operator=(const TunePin &) = delete;
 
 private:
-    TuneVersion keep_, before_;
+    TuneVersion keep_;
+    const TuneVersion *before_;  // the enclosing pin's, or null
 };
 
 // NVTX range over a host-side stage (queuing an LDE, a forest, a commit, a
