@@ -99,7 +99,7 @@ static void launch_leaf_mma(uint64_t lt, uint64_t *digests, uint64_t *caps, cons
     else launch_leaf_mma_t<H, NS, 128>(digests, caps, leaves, g, s);
 }
 
-// Tables in shared memory while every CTA can have an SM of a B200 to itself
+// Tables in shared memory while every CTA can have a multiprocessor to itself
 // (forests of 8-word leaves, 2^10: Poseidon2 159 -> 147 us, Monolith 54 -> 47).
 template <int H>
 static void launch_fold_mma(unsigned ctas, uint64_t *digests, uint64_t *caps, const MerkleGeom &g, uint32_t u0, cudaStream_t s)
@@ -107,8 +107,9 @@ static void launch_fold_mma(unsigned ctas, uint64_t *digests, uint64_t *caps, co
     constexpr uint32_t bytes = 4 * mma_table_words<H>();
     // the dynamic shared-memory opt-in is per device
     static std::atomic<uint64_t> attr_set{0};
-    int dev = 0;
-    bool copy = ctas <= 148 && cudaGetDevice(&dev) == cudaSuccess;
+    int dev = 0, sms = 0;
+    bool copy = cudaGetDevice(&dev) == cudaSuccess &&
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && ctas <= (unsigned)sms;
     const uint64_t bit = 1ULL << (dev & 63);
     if (copy && !(attr_set.load(std::memory_order_relaxed) & bit)) {
         copy = cudaFuncSetAttribute(merkle_fold_mma_kernel<H, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
