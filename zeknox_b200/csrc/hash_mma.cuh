@@ -256,12 +256,6 @@ __device__ __forceinline__ uint64_t mma_chain(uint64_t y, const uint64_t x[3])
     }
 }
 
-template <int H>
-__device__ __forceinline__ uint64_t mma_sbox(uint64_t x)
-{
-    return gl_sbox7_nc(x);
-}
-
 // Operands of a full-round layer from the state at a.  Its coefficients are
 // below 256, so byte b of an output takes byte b of the lanes alone: for column
 // pair i one k-block with bytes 2i and 2i + 1 of lanes t and 4 + t and the word
@@ -317,11 +311,11 @@ __device__ __forceinline__ void mma_rounds4(uint32_t *sm, const uint32_t *b, con
         x[j + 1] = v.y;
     }
     __syncwarp();
-    x[0] = mma_sbox<H>(x[0]);
-    x[1] = mma_sbox<H>(mma_chain<H, 1>(x[1], x));
+    x[0] = gl_sbox7_nc(x[0]);
+    x[1] = gl_sbox7_nc(mma_chain<H, 1>(x[1], x));
     if (i < 5) {  // else the coefficients of x_2 and x_3 are zero
-        x[2] = mma_sbox<H>(mma_chain<H, 2>(x[2], x));
-        x[3] = mma_sbox<H>(mma_chain<H, 3>(x[3], x));
+        x[2] = gl_sbox7_nc(mma_chain<H, 2>(x[2], x));
+        x[3] = gl_sbox7_nc(mma_chain<H, 3>(x[3], x));
     }
     if (t < NS) {
         // x_j is the operand of thread j of the quad
@@ -427,7 +421,7 @@ __device__ __forceinline__ void permute_mma(uint32_t *sm, uint32_t groups, const
 #pragma unroll
                 for (int q = 0; q < NS; q++)
 #pragma unroll
-                    for (int j = 0; j < J; j++) v[j][q] = mma_sbox<H>(v[j][q]);
+                    for (int j = 0; j < J; j++) v[j][q] = gl_sbox7_nc(v[j][q]);
             }
 #pragma unroll
             for (int j = 0; j < J; j++) mma_store_group<NS>(a + (j0 + j) * M::BLOCK, v[j]);

@@ -151,17 +151,19 @@ static void merkle_launch(uint64_t *digests, uint64_t *caps, const uint64_t *lea
     const uint32_t lg_leaves = ilog2_exact(g.n_leaves);
     const uint64_t lt = tune_get("leaf_threads." + std::to_string(H), lg_leaves, leaf_t_default<H>(g.n_leaves));
     uint64_t blocks;
-    uint64_t coop = 0;
-    if constexpr (HasMma<H>::value)
-        coop = std::min<uint64_t>(tune_get("coop_leaves." + std::to_string(H), lg_leaves, COOP_LEAVES), 1ULL << 40);
     uint32_t u0 = 0;
-    bool mma_leaf = false;
-    if constexpr (HasMma<H>::value) mma_leaf = g.leaf_size > 4;
-    if (mma_leaf) {
-        if constexpr (HasMma<H>::value) {
-            if (g.n_leaves <= coop) launch_leaf_mma<H, 1>(lt, digests, caps, leaves, g, s);
-            else if (g.n_leaves <= mid_leaves<H>() * coop) launch_leaf_mma<H, 2>(lt, digests, caps, leaves, g, s);
-            else launch_leaf_mma<H, 4>(lt, digests, caps, leaves, g, s);
+    if constexpr (HasMma<H>::value) {
+        const uint64_t coop =
+            std::min<uint64_t>(tune_get("coop_leaves." + std::to_string(H), lg_leaves, COOP_LEAVES), 1ULL << 40);
+        if (g.leaf_size <= 4) {
+            blocks = (g.n_leaves + LEAF_T - 1) / LEAF_T;
+            merkle_leaf_copy_kernel<LEAF_T><<<(unsigned)blocks, LEAF_T, 0, s>>>(leaves, digests, caps, g);
+        } else if (g.n_leaves <= coop) {
+            launch_leaf_mma<H, 1>(lt, digests, caps, leaves, g, s);
+        } else if (g.n_leaves <= mid_leaves<H>() * coop) {
+            launch_leaf_mma<H, 2>(lt, digests, caps, leaves, g, s);
+        } else {
+            launch_leaf_mma<H, 4>(lt, digests, caps, leaves, g, s);
         }
     } else if (H == HASH_POSEIDON_BN128 && g.leaf_size > 4 &&
                g.n_leaves <= tune_get("coop_leaves.2", lg_leaves, BN128_COOP_LEAVES)) {

@@ -10,7 +10,8 @@
 // Kernel structure (B200-first instead of one launch per level):
 //   * leaf kernel: one thread per leaf runs the sponge with the state in
 //     registers (nothing else, so no warp idles on a barrier), or a warp 8, 16
-//     or 32 leaves with the linear layers on the tensor cores;
+//     or 32 leaves with the linear layers on the tensor cores; rows of up to
+//     4 words are copied;
 //   * level kernel: one thread per node of one level, for the wide levels
 //     just above the leaves (and for levels a tail CTA cannot hold);
 //   * fold kernel: each CTA folds T consecutive nodes log2(T) levels up in
@@ -55,6 +56,17 @@ __device__ __forceinline__ void leaf_hash(const uint64_t *__restrict__ row, uint
     hash_one<H>(row, len, out);
 }
 
+// Where leaf i's digest goes: a digest, or with caps == leaves the cap (digests
+// untouched).  Null when the checked build finds it or the leaf out of range.
+__device__ __forceinline__ uint64_t *merkle_leaf_dst(uint64_t i, uint64_t *digests, uint64_t *caps, const MerkleGeom &g)
+{
+    if (g.sub_leaves == 1 ? !ZK_IN_BOUNDS(4 * i + 3, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)
+                          : !ZK_IN_BOUNDS(4 * merkle_node_index(g, i, 0) + 3, merkle_digest_words(g), OOB_MERKLE_DIGEST))
+        return nullptr;
+    if (g.leaf_size && !ZK_IN_BOUNDS((i + 1) * g.leaf_size - 1, merkle_leaf_words(g), OOB_MERKLE_LEAF)) return nullptr;
+    return g.sub_leaves == 1 ? caps + 4 * i : digests + 4 * merkle_node_index(g, i, 0);
+}
+
 // Leaf digests only: one thread per leaf, no shared memory, no barriers, so
 // every warp stays on the hash for the whole kernel.
 template <int H, int T>
@@ -63,12 +75,8 @@ __device__ __forceinline__ void merkle_leaf_body(const uint64_t *__restrict__ le
 {
     const uint64_t i = (uint64_t)blockIdx.x * T + threadIdx.x;
     if (i >= g.n_leaves) return;
-    // caps == leaves: the leaf hashes are the caps, digests untouched
-    uint64_t *dst = g.sub_leaves == 1 ? caps + 4 * i : digests + 4 * merkle_node_index(g, i, 0);
-    if (g.sub_leaves == 1 ? !ZK_IN_BOUNDS(4 * i + 3, 4 * (uint64_t)g.n_caps, OOB_MERKLE_CAP)
-                          : !ZK_IN_BOUNDS(4 * merkle_node_index(g, i, 0) + 3, merkle_digest_words(g), OOB_MERKLE_DIGEST))
-        return;
-    if (g.leaf_size && !ZK_IN_BOUNDS((i + 1) * g.leaf_size - 1, merkle_leaf_words(g), OOB_MERKLE_LEAF)) return;
+    uint64_t *dst = merkle_leaf_dst(i, digests, caps, g);
+    if (!dst) return;
     uint64_t d[4];
     if (H == HASH_KECCAK && g.leaf_size < 4) {
         // Keccak copies a < 4-word leaf and leaves the other digest words as
@@ -87,6 +95,20 @@ __global__ void __launch_bounds__(T)
                        MerkleGeom g)
 {
     merkle_leaf_body<H, T>(leaves, digests, caps, g);
+}
+
+// Leaves of at most 4 words under Plonky2's sponge: the words themselves, zero padded.
+template <int T>
+__global__ void __launch_bounds__(T)
+    merkle_leaf_copy_kernel(const uint64_t *__restrict__ leaves, uint64_t *__restrict__ digests, uint64_t *__restrict__ caps,
+                            MerkleGeom g)
+{
+    const uint64_t i = (uint64_t)blockIdx.x * T + threadIdx.x;
+    if (i >= g.n_leaves) return;
+    uint64_t *dst = merkle_leaf_dst(i, digests, caps, g);
+    if (!dst) return;
+#pragma unroll
+    for (uint64_t q = 0; q < 4; q++) dst[q] = q < g.leaf_size ? leaves[i * g.leaf_size + q] : 0;
 }
 
 // Folds stored digests upwards from height u0 (0 = leaf digests): each CTA
