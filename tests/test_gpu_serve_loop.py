@@ -217,3 +217,26 @@ def test_corner_columns_through_loop_match_oracle(values, h):
         assert np.array_equal(device_words(r.digests, n_dig * 4).reshape(-1, 4), d)
         assert np.array_equal(ch.numpy().view(np.uint64).reshape(-1, 4), c)
         srv.release(t)
+
+
+LEAF_COOP = 3  # stage kind: leaf digests, one leaf per group of four threads
+
+
+@pytest.mark.parametrize("h", [0, 3])
+def test_leaf_form_is_the_loops_own(h):
+    """coop_leaves is measured on the standalone forests' tensor-core kernels; the
+    loop's four-threads-per-leaf stage keeps its own crossover of 2^13 leaves."""
+    zk.tune_set("coop_leaves.%d" % h, 1 << 12)
+    try:
+        with zk.Server(0, 1 << 28, 2, device_loop=True) as srv:
+            for lg, coop in ((10, True), (11, False)):
+                inp = to_dev(O.field_data(lg + h, 9 << lg))
+                caps = torch.empty(16 * 4, dtype=torch.int64).pin_memory()
+                t = srv.submit(lg, 3, 9, 4, h, inp, caps)
+                assert srv.wait(t).status == 2
+                assert any(kind == LEAF_COOP for kind, _ in srv.trace(t)) == coop
+                srv.release(t)
+    finally:
+        zk.tune_clear()
+        if zk.os.path.exists(zk.TUNE_TABLE):
+            zk.tune_load(zk.TUNE_TABLE)

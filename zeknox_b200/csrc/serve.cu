@@ -376,7 +376,10 @@ struct Server {
         };
         const uint32_t lg_leaves = ilog2_exact(n_leaves);
         const std::string h = std::to_string(hash);
-        if (coop && n_leaves <= tune_get("coop_leaves." + h, lg_leaves, 1ULL << 13))
+        // four threads a leaf up to 2^13 leaves (0.46 against 0.76 ms at 2^13 x
+        // 84 Poseidon, slower from 2^14 on); the knob coop_leaves is the
+        // crossover of merkle.cu's tensor-core forms, another one
+        if (coop && n_leaves <= (1ULL << 13))
             stage(LS_LEAF_COOP, 0, (n_leaves + LOOP_THREADS / 4 - 1) / (LOOP_THREADS / 4));
         else
             stage(LS_LEAF, 0, (n_leaves + LOOP_THREADS - 1) / LOOP_THREADS);
