@@ -317,7 +317,7 @@ def run_ours(args, rank, world):
     tr_bytes = 16 * N * COLS
 
     def time_transpose(form):
-        zk.tune_set("transpose_bulk", form)
+        zk.tune_set("transpose_bulk", form, lg=LG_N + RATE)  # the table has an entry of this size
         ms = []
         for s in range(reps + 1):
             flush.fill_(s & 0xFF)
@@ -334,7 +334,7 @@ def run_ours(args, rank, world):
         tr_16 = time_transpose(0)  # 16-byte loads through registers
         tr_t = time_transpose(zk.TRANSPOSE_AUTO)  # bulk-async copies into shared-memory stages (the default)
     finally:
-        zk.tune_set("transpose_bulk", zk.TRANSPOSE_AUTO)
+        zk.tune_set("transpose_bulk", zk.TRANSPOSE_AUTO, lg=LG_N + RATE)
     roofline_transpose = {"bound": "hbm", "kernel": "transpose_rev_bulk_kernel (compute_transpose_rev, 256 x 2^18)",
                           "achieved": tr_bytes / tr_t / 1e9, "peak": hbm, "unit": "GB/s",
                           "frac": tr_bytes / tr_t / 1e9 / hbm, "algorithmic_bytes": tr_bytes, "ms": tr_t * 1e3,

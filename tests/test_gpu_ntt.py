@@ -126,12 +126,12 @@ def test_transpose_rev_bulk_and_plain_forms(lg, b):
     outs = []
     try:
         for form in (1, 2, 3, 4, 5, 6, 7, 8, 0):
-            zk.tune_set("transpose_bulk", form)
+            zk.tune_set("transpose_bulk", form, lg=lg)  # the table has entries of some sizes
             out = torch.zeros(b << lg, dtype=torch.int64, device="cuda")
             zk.transpose_rev_batch(0, out, src, lg, b)
             outs.append(out)
     finally:
-        zk.tune_set("transpose_bulk", zk.TRANSPOSE_AUTO)
+        zk.tune_set("transpose_bulk", zk.TRANSPOSE_AUTO, lg=lg)
     assert np.array_equal(to_np(outs[0]), exp)
     for o in outs[1:]:
         assert torch.equal(outs[0], o)
