@@ -220,14 +220,23 @@ RustError zeknox_server_destroy(void *server);
 
 /* ---- Tuning (written by zeknox_b200/autotune.py; no reference counterpart)
  * Knobs, each optionally per log2 size (lg = 0xFFFFFFFF: any size):
- *   "leaf_threads.<hash_type>"  Merkle leaf kernel CTA size, 64/128/256 (lg = log2 leaves)
+ *   "leaf_threads.<hash_type>"  Merkle leaf kernel CTA size (lg = log2 leaves): 32/64/128 for Poseidon,
+ *                               Poseidon2 and Monolith (any other value: 128), 64/128/256 for the rest
  *   "lde_chunk_mib"             fused-LDE column chunk budget in MiB (lg = log2 N)
  *   "lde_host_chunk_mib"        the same for inputs in host memory (copies overlap the chunks)
  *   "lde_last_logr"             radix exponent of the fused LDE's row-output pass, 1..8 (lg = log2 n)
  *   "wide_level_nodes.<hash_type>"  Merkle levels at least this wide run node-parallel (lg = log2 leaves)
- *   "coop_leaves.<hash_type>"   forests of at most this many leaves hash them with four threads per
- *                               permutation (Poseidon, Poseidon2; lg = log2 leaves)
- * Unset knobs keep the built-in defaults.  Results never depend on the knobs. */
+ *   "coop_leaves.<hash_type>"   forests of at most this many leaves hash them in the latency form (lg =
+ *                               log2 leaves): 8 leaves per warp for Poseidon, Poseidon2 and Monolith (16
+ *                               up to four times as many, Monolith 32 times, else 32), five threads per
+ *                               permutation for Poseidon-BN128
+ *   "ntt_split_logr"            largest pass, 2^1..2^10 points, of a column-output transform; 0: built in
+ *                               (lg = log2 n)
+ *   "transpose_bulk"            transpose form: 0 through registers, 1..8 bulk-copy tile shapes, 9 by the
+ *                               column count (lg = log2 n)
+ * Unset knobs keep the built-in defaults.  Results never depend on the knobs.
+ * Any thread may change them at any time: a call uses the table as it was when
+ * the call began, a server request as it was when it was submitted. */
 RustError zeknox_tune_set(const char *name, uint32_t lg, uint64_t value);
 RustError zeknox_tune_clear(void);
 /* Value a knob has for log2 size lg (the size-free entry, else dflt). */

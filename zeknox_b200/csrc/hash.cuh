@@ -444,14 +444,11 @@ ZK_HD void keccak_f(uint64_t st[25])
 
 // The matrix layers' dot products of five terms as one reduction (1) or as
 // five fr_mul and four fr_add (0).  Both give the same canonical values.  The
-// first, with its product and reduction steps out of line (one copy of their
-// code: inlined at the call sites they stalled the leaf kernel on instruction
-// fetch), measured 1.20x on a 2^20 x 135 Poseidon-BN128 forest (450 ms against
-// 540) and 1.64x on a 2^14 x 135 one (18.0 against 29.5), with 128-thread leaf
-// CTAs; it is the default.  The device-resident request loop compiles the
-// second: built with the first (inlined), its kernel's register frame grew
-// and its transform stages ran 14% slower (2^20 x 256 LDE: 61.0 ms against
-// 53.7), because all stages share that kernel's 64-register budget.  Units
+// first is the host's form.  The second is the only one a device unit compiles,
+// the device-resident request loop's: built with the first, its kernel's
+// register frame grew and its transform stages ran 14% slower (2^20 x 256 LDE:
+// 61.0 ms against 53.7), because all stages share that kernel's 64-register
+// budget.  The Merkle kernels run neither but bn254_29.cuh.  Units
 // built with different settings hold different bodies of the functions
 // below; they are force-inlined (no out-of-line host symbol), the steps they
 // call are file-local, and device code is not linked across units.
