@@ -214,10 +214,20 @@ void DeviceCtx::sync()
     check_waits();
 }
 
+// Lets this thread make calls that a stream capture would refuse.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { ZK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode)); }
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 unsigned *DeviceCtx::wait_status()
 {
     if (!wait_status_dev) {
         void *h = nullptr;
+        // the first user may be a transpose that this or another thread records
+        // into a graph: the allocation is no part of it
+        RelaxedCapture relaxed;
         ZK_CUDA(cudaHostAlloc(&h, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable));
         *(volatile unsigned *)h = 0;
         void *d = nullptr;
