@@ -235,8 +235,8 @@ RustError zeknox_server_destroy(void *server);
  *   "transpose_bulk"            transpose form: 0 through registers, 1..8 bulk-copy tile shapes, 9 by the
  *                               column count (lg = log2 n)
  * Unset knobs keep the built-in defaults.  Results never depend on the knobs.
- * Any thread may change them at any time: a call uses the table as it was when
- * the call began, a server request as it was when it was submitted. */
+ * Any thread may change them at any time: a call reads one version of the
+ * table throughout, a server request that of its submission. */
 RustError zeknox_tune_set(const char *name, uint32_t lg, uint64_t value);
 RustError zeknox_tune_clear(void);
 /* Value a knob has for log2 size lg (the size-free entry, else dflt). */

@@ -35,6 +35,7 @@ int main(int, char **argv)
             TunePin inner;  // keeps the enclosing pin's version
             CHECK(tune_get("ntt_split_logr", 12, 0) == 9);
         }
+        CHECK(tune_get("ntt_split_logr", 12, 0) == 9);
         tune_set("ntt_split_logr", TUNE_ANY, 8);  // this thread's own change too
         CHECK(tune_get("ntt_split_logr", 13, 0) == 9 && tune_generation() == gen);
     }
@@ -46,6 +47,20 @@ int main(int, char **argv)
         CHECK(tune_get("ntt_split_logr", 12, 0) == 9 && tune_generation() == gen);
     }
     CHECK(tune_get("ntt_split_logr", 12, 0) == 0);
+    {
+        TunePin outer;  // reads nothing before the inner pin does
+        {
+            TunePin inner;
+            CHECK(tune_get("ntt_split_logr", 12, 0) == 0);
+            {
+                TunePin request(queued);
+                CHECK(tune_get("ntt_split_logr", 12, 0) == 9);
+            }
+        }
+        tune_set("ntt_split_logr", 12, 5);
+        CHECK(tune_get("ntt_split_logr", 12, 0) == 0);
+    }
+    CHECK(tune_get("ntt_split_logr", 12, 0) == 5);
     // readers of one version see one value however often it changes
     bool same = true, stop = false;
     std::thread writer([&] {

@@ -43,7 +43,7 @@ struct TuneTable {
 
 static std::mutex g_tune_mu;
 static TuneVersion g_tune = std::make_shared<const TuneTable>();  // the newest
-static thread_local const TuneVersion *t_pinned = nullptr;  // the innermost pin's
+static thread_local TunePin *t_pin = nullptr;  // the one in force
 
 // The newest table with `change` made to it becomes the newest.
 template <class F>
@@ -71,24 +71,36 @@ static void tune_env_load()
     }
 }
 
-TuneVersion tune_version()
+static TuneVersion newest_version()
 {
-    if (t_pinned) return *t_pinned;
     std::call_once(g_tune_env_once, tune_env_load);
     std::lock_guard<std::mutex> lk(g_tune_mu);
     return g_tune;
 }
 
-TunePin::TunePin(TuneVersion v) : keep_(std::move(v)), before_(t_pinned) { t_pinned = &keep_; }
-TunePin::~TunePin() { t_pinned = before_; }
+TunePin::TunePin() : before_(t_pin)
+{
+    if (!t_pin) t_pin = this;
+}
+TunePin::TunePin(TuneVersion v) : keep_(std::move(v)), before_(t_pin) { t_pin = this; }
+TunePin::~TunePin() { t_pin = before_; }
+
+// The version of the pin in force.
+const TuneVersion &tune_pinned()
+{
+    if (!t_pin->keep_) t_pin->keep_ = newest_version();
+    return t_pin->keep_;
+}
+
+TuneVersion tune_version() { return t_pin ? tune_pinned() : newest_version(); }
 
 uint64_t tune_generation() { return tune_version()->generation; }
 
 uint64_t tune_get(const std::string &name, uint32_t lg, uint64_t dflt)
 {
     TuneVersion newest;
-    if (!t_pinned) newest = tune_version();
-    const auto &knobs = (t_pinned ? *t_pinned : newest)->knobs;
+    if (!t_pin) newest = newest_version();
+    const auto &knobs = (t_pin ? tune_pinned() : newest)->knobs;
     auto it = knobs.find({name, lg});
     if (it != knobs.end()) return it->second;
     it = knobs.find({name, TUNE_ANY});
